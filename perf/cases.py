@@ -295,7 +295,7 @@ class _Gaussian:
         # (a tensor divisor: a plain number is turned into a multiplication, which may round into the next cell)
         cell = torch.floor(x.view(3, N) / torch.full_like(x[:1], h) + (0.5 if P % 2 else 0.0))
         steps = lo + torch.arange(P, device=x.device)
-        u = (x.view(3, N) - cell * h)[..., None] - steps * h
+        u = (x.view(3, N) - cell * h)[..., None] - steps.double() * h
         self.index = (cell.long()[..., None] + steps) % M
         self.weight = torch.exp(-self.c * u * u)
         self.slope = -self.c * u * self.weight
