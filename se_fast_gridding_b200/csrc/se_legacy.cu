@@ -307,17 +307,15 @@ __global__ void k_base_gaussian(double* zs, ParamsDev p)
     zs[t] = p.d * exp(-p.c * (a * a + b * b + e * e));
 }
 
-// One particle's expansion, SE_fgg.c:539-621 (3P), :625-722 (force),
-// :727-819 (2P: z free, offset a), :823-916 (1P: x and y free, offsets a
-// and b); q folded into zx.  Returns the padded corner index.
-__device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int periodicity,
-                          double* zx, double* zy, double* zz, double* zfx, double* zfy,
-                          double* zfz)
+// One particle's stencil: the offset t0 of the position from the nearest
+// (odd P) or lower (even P) grid point per axis, and the padded corner index.
+__device__ __forceinline__ int expand_corner(const double xn[3], const ParamsDev& p,
+                                             int periodicity, double t0[3])
 {
-    const int P = p.P, ph = p.P_half;
-    const bool odd = P & 1;
-    double t0[3];
+    const int ph = p.P_half;
+    const bool odd = p.P & 1;
     int first[3];
+#pragma unroll
     for (int d = 0; d < 3; d++) {
         const bool sh = (periodicity == 2 && d == 2) || (periodicity == 1 && d < 2);
         const double s = sh ? (periodicity == 1 && d == 1 ? p.b : p.a) + p.h / 2 : 0.0;
@@ -326,6 +324,22 @@ __device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int 
         first[d] = odd ? cell - ph : cell - (ph - 1);
         t0[d] = sh ? xn[d] - (cell * p.h + s) : xn[d] - p.h * cell;
     }
+    if (periodicity == 1)   // the free x and y corners are not shifted (:912-915)
+        return (first[0] * p.npdims[1] + first[1]) * p.npdims[2] + first[2] + ph;
+    const int kz = periodicity == 2 ? first[2] : first[2] + ph;
+    return ((first[0] + ph) * p.npdims[1] + first[1] + ph) * p.npdims[2] + kz;
+}
+
+// One particle's expansion, SE_fgg.c:539-621 (3P), :625-722 (force),
+// :727-819 (2P: z free, offset a), :823-916 (1P: x and y free, offsets a
+// and b); q folded into zx.  Returns the padded corner index.
+__device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int periodicity,
+                          double* zx, double* zy, double* zz, double* zfx, double* zfy,
+                          double* zfz)
+{
+    const int P = p.P;
+    double t0[3];
+    const int corner = expand_corner(xn, p, periodicity, t0);
     const double z3 = exp(-p.c * (t0[0] * t0[0] + t0[1] * t0[1] + t0[2] * t0[2])) * q;
     double* z[3] = {zx, zy, zz};
     double* zf[3] = {zfx, zfy, zfz};
@@ -341,81 +355,192 @@ __device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int 
             for (int i = 0; i < P; i++) zf[d][i] = -p.c * (t0[d] - (p.lo + i) * p.h);
     }
     for (int i = 0; i < P; i++) zx[i] *= z3;
-    if (periodicity == 1)   // the free x and y corners are not shifted (:912-915)
-        return (first[0] * p.npdims[1] + first[1]) * p.npdims[2] + first[2] + ph;
-    const int kz = periodicity == 2 ? first[2] : first[2] + ph;
-    return ((first[0] + ph) * p.npdims[1] + first[1] + ph) * p.npdims[2] + kz;
+    return corner;
 }
 
-// SE_fgg.c:920-963 (q = 1)
-__global__ void k_expand_all(ParamsDev p, const double* __restrict__ x, int periodicity,
-                             double* zx, double* zy, double* zz, double* zfx, double* zfy,
-                             double* zfz, int* idx)
+// SE_fgg.c:920-963 (q = 1).  A warp expands 32 particles, one per lane; the
+// rows go through shared memory so that they are stored P consecutive values
+// at a time (stored by their own lanes, P values apart: 30,000 particles, P =
+// 16, force, B200: 26 -> 15 us).
+constexpr int EXPAND_WARPS = 4;
+
+__global__ void __launch_bounds__(EXPAND_WARPS * 32) k_expand_all(
+    ParamsDev p, const double* __restrict__ x, int periodicity, double* zx, double* zy, double* zz,
+    double* zfx, double* zfy, double* zfz, int* idx)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.N) return;
+    __shared__ double row[EXPAND_WARPS][32][SE_P_MAX + 1];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (blockIdx.x * EXPAND_WARPS + w) * 32, n = min(n0 + lane, p.N - 1);
+    const int cnt = min(32, p.N - n0);
+    if (cnt <= 0) return;
     const double xn[3] = {x[n], x[n + p.N], x[n + 2 * p.N]};
-    const long long o = (long long)n * p.P;
-    idx[n] = expand_one(xn, 1.0, p, periodicity, zx + o, zy + o, zz + o,
-                        zfx ? zfx + o : nullptr, zfy ? zfy + o : nullptr,
-                        zfz ? zfz + o : nullptr);
+    double t0[3];
+    double* zs[3] = {zx, zy, zz};
+    double* zf[3] = {zfx, zfy, zfz};
+    const int corner = expand_corner(xn, p, periodicity, t0);
+    if (lane < cnt) idx[n] = corner;
+    const double z3 = exp(-p.c * (t0[0] * t0[0] + t0[1] * t0[1] + t0[2] * t0[2]));
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const double base = exp(2 * p.c * p.h * t0[d]);
+        double v = pow(base, (double)p.lo);
+        row[w][lane][0] = d == 0 ? v * z3 : v;
+        for (int i = 1; i < p.P; i++) {
+            v *= base;
+            row[w][lane][i] = d == 0 ? v * z3 : v;
+        }
+        __syncwarp();
+        for (int r = 0; r < cnt; r++) {
+            const double t = __shfl_sync(0xffffffffu, t0[d], r);
+            if (lane < p.P) {
+                const long long o = (long long)(n0 + r) * p.P + lane;
+                zs[d][o] = row[w][r][lane];
+                if (zf[d]) zf[d][o] = -p.c * (t - (p.lo + lane) * p.h);
+            }
+        }
+        __syncwarp();
+    }
 }
 
-// Scatter of one particle's P^3 stencil per CTA.  force_order selects the
-// product order of SE_fgg.c:4964-5009 instead of :3983-4028.
-__global__ void k_grid_split(double* H, const double* __restrict__ q,
-                             const double* __restrict__ zs, const double* __restrict__ zx,
-                             const double* __restrict__ zy, const double* __restrict__ zz,
-                             const int* __restrict__ idx, ParamsDev p, int force_order)
+// The walk over one particle's P^3 stencil by a warp, for the scatter and
+// gather kernels below.  Lane l takes z entry k = l % P of the y rows j =
+// l / P + m R, R = 32 / P, of every x plane: neighbouring lanes on
+// neighbouring cells, no index divided inside the loops (a division of the
+// linear index by P and P^2 for every cell bound these kernels before: P =
+// 16, 30,000 particles, B200: scatter 428 -> 265 us, force gather 514 -> 370
+// us).  The rows go eight at a time, with their y factors in registers for
+// all x planes.
+constexpr int STENCIL_ROWS = 8;
+
+struct StencilLane {
+    int k, j0, R;
+    bool on;
+    __device__ __forceinline__ StencilLane(int P)
+    {
+        const int lane = threadIdx.x & 31;
+        R = max(32 / P, 1);
+        k = lane % P;
+        j0 = lane / P;
+        on = j0 < R;
+    }
+};
+
+// H[cell] += zs[cell] zz[k] (q zx[i] zy[j]), or the product order of
+// SE_fgg.c:4964-5009 (force_order) instead of that of :3983-4028.
+__device__ __forceinline__ void scatter_stencil(double* H, long long base, int P, int n1, int n2,
+                                                const double* __restrict__ zs, const double* zx,
+                                                const double* zy, const double* zz, double q,
+                                                int force_order)
 {
-    const int n = blockIdx.x;
-    const int P = p.P;
-    const long long o = (long long)n * P;
-    const double qn = q[n];
+    const StencilLane L(P);
+    if (!L.on) return;
+    const double zk = zz[L.k];
+    for (int jc = L.j0; jc < P; jc += STENCIL_ROWS * L.R) {
+        double y[STENCIL_ROWS];
+#pragma unroll
+        for (int m = 0; m < STENCIL_ROWS; m++) y[m] = jc + m * L.R < P ? zy[jc + m * L.R] : 0.0;
+        const double* z = zs + jc * P + L.k;
+        double* h = H + base + (long long)jc * n2 + L.k;
+        for (int i = 0; i < P; i++, z += P * P, h += (long long)n1 * n2) {
+            const double x = force_order ? zx[i] : q * zx[i];
+#pragma unroll
+            for (int m = 0; m < STENCIL_ROWS; m++) {
+                if (jc + m * L.R >= P) break;
+                double v = z[m * L.R * P] * zk * (x * y[m]);
+                if (force_order) v *= q;
+                atomicAdd(h + (long long)m * L.R * n2, v);
+            }
+        }
+    }
+}
+
+// This lane's part of a[0] = sum H zs zz zx zy and, with FORCE, a[1..3] = the
+// same sums times zfx[i], zfy[j], zfz[k].
+template <bool FORCE>
+__device__ __forceinline__ void gather_stencil(const double* __restrict__ H, long long base, int P, int n1,
+                                               int n2, const double* __restrict__ zs, const double* zx,
+                                               const double* zy, const double* zz, const double* zfx,
+                                               const double* zfy, const double* zfz, double (&a)[4])
+{
+    const StencilLane L(P);
+    a[0] = a[1] = a[2] = a[3] = 0.0;
+    if (!L.on) return;
+    for (int jc = L.j0; jc < P; jc += STENCIL_ROWS * L.R) {
+        double y[STENCIL_ROWS], fy[STENCIL_ROWS];
+#pragma unroll
+        for (int m = 0; m < STENCIL_ROWS; m++) {
+            const int j = jc + m * L.R;
+            y[m] = j < P ? zy[j] : 0.0;
+            fy[m] = FORCE && j < P ? y[m] * zfy[j] : 0.0;
+        }
+        const double* z = zs + jc * P + L.k;
+        const double* h = H + base + (long long)jc * n2 + L.k;
+        for (int i = 0; i < P; i++, z += P * P, h += (long long)n1 * n2) {
+            double s = 0.0, sy = 0.0;
+#pragma unroll
+            for (int m = 0; m < STENCIL_ROWS; m++) {
+                if (jc + m * L.R >= P) break;
+                const double v = h[(long long)m * L.R * n2] * z[m * L.R * P];
+                s = fma(v, y[m], s);
+                if (FORCE) sy = fma(v, fy[m], sy);
+            }
+            s *= zx[i];
+            a[0] += s;
+            if (FORCE) {
+                a[1] = fma(s, zfx[i], a[1]);
+                a[2] = fma(sy, zx[i], a[2]);
+            }
+        }
+    }
+    const double zk = zz[L.k];
+    a[0] *= zk;
+    if (FORCE) {
+        a[1] *= zk;
+        a[2] *= zk;
+        a[3] = a[0] * zfz[L.k];
+    }
+}
+
+// Scatter of one particle's P^3 stencil per warp.
+constexpr int SCATTER_WARPS = 8;
+
+__global__ void __launch_bounds__(SCATTER_WARPS * 32) k_grid_split(
+    double* H, const double* __restrict__ q, const double* __restrict__ zs, const double* __restrict__ zx,
+    const double* __restrict__ zy, const double* __restrict__ zz, const int* __restrict__ idx, ParamsDev p,
+    int force_order)
+{
+    const int n = blockIdx.x * SCATTER_WARPS + (threadIdx.x >> 5);
+    if (n >= p.N) return;
+    const long long o = (long long)n * p.P;
     const long long base = idx[n];
     if (!stencil_in_bounds(base, p)) {
-        if (threadIdx.x == 0) atomicOr(&g_legacy_err, 1);
+        if ((threadIdx.x & 31) == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    const int n1 = p.npdims[1], n2 = p.npdims[2];
-    for (int s = threadIdx.x; s < P * P * P; s += blockDim.x) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        double v;
-        if (force_order) {
-            const double cij = zx[o + i] * zy[o + j];
-            v = zs[s] * zz[o + k] * cij * qn;
-        } else {
-            const double cij = qn * zx[o + i] * zy[o + j];
-            v = zs[s] * zz[o + k] * cij;
-        }
-        atomicAdd(H + base + ((long long)i * n1 + j) * n2 + k, v);
-    }
+    scatter_stencil(H, base, p.P, p.npdims[1], p.npdims[2], zs, zx + o, zy + o, zz + o, q[n], force_order);
 }
 
 // SE_fgg.c:3866-3914: expansion with the charge, then the same scatter
-__global__ void k_grid_vanilla(double* H, const double* __restrict__ x,
-                               const double* __restrict__ q, const double* __restrict__ zs,
-                               ParamsDev p, int periodicity)
+__global__ void __launch_bounds__(SCATTER_WARPS * 32) k_grid_vanilla(
+    double* H, const double* __restrict__ x, const double* __restrict__ q, const double* __restrict__ zs,
+    ParamsDev p, int periodicity)
 {
-    __shared__ double z[3][SE_P_MAX];
-    __shared__ int c0;
-    const int n = blockIdx.x;
-    const int P = p.P;
-    if (threadIdx.x == 0) {
+    __shared__ double zsm[SCATTER_WARPS][3][SE_P_MAX];
+    __shared__ int c0s[SCATTER_WARPS];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = blockIdx.x * SCATTER_WARPS + w;
+    if (n >= p.N) return;
+    double(&z)[3][SE_P_MAX] = zsm[w];
+    if (lane == 0) {
         const double xn[3] = {x[n], x[n + p.N], x[n + 2 * p.N]};
-        c0 = expand_one(xn, q[n], p, periodicity, z[0], z[1], z[2], nullptr, nullptr, nullptr);
+        c0s[w] = expand_one(xn, q[n], p, periodicity, z[0], z[1], z[2], nullptr, nullptr, nullptr);
     }
-    __syncthreads();
-    if (!stencil_in_bounds(c0, p)) {
-        if (threadIdx.x == 0) atomicOr(&g_legacy_err, 1);
+    __syncwarp();
+    if (!stencil_in_bounds(c0s[w], p)) {
+        if (lane == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    const int n1 = p.npdims[1], n2 = p.npdims[2];
-    for (int s = threadIdx.x; s < P * P * P; s += blockDim.x) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        const double cij = z[0][i] * z[1][j];
-        atomicAdd(H + c0 + ((long long)i * n1 + j) * n2 + k, zs[s] * z[2][k] * cij);
-    }
+    scatter_stencil(H, c0s[w], p.P, p.npdims[1], p.npdims[2], zs, z[0], z[1], z[2], 1.0, 0);
 }
 
 // SE_fgg.c:327-352 / :357-382 / :387-411 as a gather: each periodic cell adds
@@ -501,13 +626,9 @@ __global__ void k_int_split(double* phi, const double* __restrict__ H,
         if (lane == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    double acc = 0;
-    for (int s = lane; s < P * P * P; s += 32) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        const double cij = zx[o + i] * zy[o + j];
-        acc += H[base + ((long long)i * n1 + j) * n2 + k] * zs[s] * zz[o + k] * cij;
-    }
-    acc = warp_sum_d(acc);
+    double a[4];
+    gather_stencil<false>(H, base, P, n1, n2, zs, zx + o, zy + o, zz + o, nullptr, nullptr, nullptr, a);
+    const double acc = warp_sum_d(a[0]);
     if (lane == 0) phi[m] = accumulate ? phi[m] + h3 * acc : h3 * acc;
 }
 
@@ -533,13 +654,9 @@ __global__ void k_int_vanilla(double* phi, const double* __restrict__ H,
         if (lane == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    double acc = 0;
-    for (int s = lane; s < P * P * P; s += 32) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        const double cij = z[w][0][i] * z[w][1][j];
-        acc += H[base + ((long long)i * n1 + j) * n2 + k] * zs[s] * z[w][2][k] * cij;
-    }
-    acc = warp_sum_d(acc);
+    double a[4];
+    gather_stencil<false>(H, base, P, n1, n2, zs, z[w][0], z[w][1], z[w][2], nullptr, nullptr, nullptr, a);
+    const double acc = warp_sum_d(a[0]);
     if (lane == 0) phi[m] = h3 * acc;
 }
 
@@ -563,18 +680,9 @@ __global__ void k_int_split_force(double* force, const double* __restrict__ q,
         return;
     }
     const double qm = q[m];
-    double f0 = 0, f1 = 0, f2 = 0;
-    for (int s = lane; s < P * P * P; s += 32) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        const double cij = zx[o + i] * zy[o + j];
-        const double t = H[base + ((long long)i * n1 + j) * n2 + k] * zs[s] * zz[o + k] * cij * qm;
-        f0 += t * zfx[o + i];
-        f1 += t * zfy[o + j];
-        f2 += t * zfz[o + k];
-    }
-    f0 = warp_sum_d(f0);
-    f1 = warp_sum_d(f1);
-    f2 = warp_sum_d(f2);
+    double a[4];
+    gather_stencil<true>(H, base, P, n1, n2, zs, zx + o, zy + o, zz + o, zfx + o, zfy + o, zfz + o, a);
+    const double f0 = warp_sum_d(a[1]) * qm, f1 = warp_sum_d(a[2]) * qm, f2 = warp_sum_d(a[3]) * qm;
     if (lane == 0) {
         force[m] = h3 * f0;
         force[m + p.N] = h3 * f1;
@@ -604,18 +712,9 @@ __global__ void k_int_force_vanilla(double* force, const double* __restrict__ H,
         if (lane == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    double f0 = 0, f1 = 0, f2 = 0;
-    for (int s = lane; s < P * P * P; s += 32) {
-        const int i = s / (P * P), j = (s / P) % P, k = s % P;
-        const double cij = z[w][0][i] * z[w][1][j];
-        const double t = H[base + ((long long)i * n1 + j) * n2 + k] * zs[s] * z[w][2][k] * cij;
-        f0 += t * z[w][3][i];
-        f1 += t * z[w][4][j];
-        f2 += t * z[w][5][k];
-    }
-    f0 = warp_sum_d(f0);
-    f1 = warp_sum_d(f1);
-    f2 = warp_sum_d(f2);
+    double a[4];
+    gather_stencil<true>(H, base, P, n1, n2, zs, z[w][0], z[w][1], z[w][2], z[w][3], z[w][4], z[w][5], a);
+    const double f0 = warp_sum_d(a[1]), f1 = warp_sum_d(a[2]), f2 = warp_sum_d(a[3]);
     if (lane == 0) {
         force[m] = h3 * f0;
         force[m + p.N] = h3 * f1;
@@ -731,7 +830,8 @@ static int do_expand(SE_FGG_work* w, const SE_state* st, const SE_FGG_params* p,
     double* fz = force ? (double*)s.use(w->zfz, NP * 8, false, true) : nullptr;
     int* idx = (int*)s.use(w->idx, 4 * (size_t)p->N, false, true);
     SE_TRY(s.copy_in());
-    k_expand_all<<<blocks(p->N, 128), 128>>>(to_dev(p), x, periodicity, zx, zy, zz, fx, fy, fz, idx);
+    k_expand_all<<<blocks(p->N, EXPAND_WARPS * 32), EXPAND_WARPS * 32>>>(
+        to_dev(p), x, periodicity, zx, zy, zz, fx, fy, fz, idx);
     return s.finish();
 }
 
@@ -751,7 +851,8 @@ static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params
     const double* zz = (const double*)s.use(w->zz, NP * 8, true, false);
     const int* idx = (const int*)s.use(w->idx, 4 * (size_t)p->N, true, false);
     SE_TRY(s.copy_in());
-    k_grid_split<<<p->N, 256>>>(H, q, zs, zx, zy, zz, idx, to_dev(p), force_order);
+    k_grid_split<<<blocks(p->N, SCATTER_WARPS), SCATTER_WARPS * 32>>>(
+        H, q, zs, zx, zy, zz, idx, to_dev(p), force_order);
     return s.finish();
 }
 
@@ -767,7 +868,8 @@ static int do_grid_vanilla(SE_FGG_work* w, const SE_state* st, const SE_FGG_para
     const double* q = (const double*)s.use(st->q, 8 * (size_t)p->N, true, false);
     const double* zs = (const double*)s.use(w->zs, P3 * 8, true, false);
     SE_TRY(s.copy_in());
-    k_grid_vanilla<<<p->N, 256>>>(H, x, q, zs, to_dev(p), periodicity_default());
+    k_grid_vanilla<<<blocks(p->N, SCATTER_WARPS), SCATTER_WARPS * 32>>>(H, x, q, zs, to_dev(p),
+                                                                               periodicity_default());
     return s.finish();
 }
 
