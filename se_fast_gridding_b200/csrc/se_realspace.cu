@@ -10,14 +10,15 @@
 //               order for every target;
 //   cell list   0 < rc <= L/2 with at least 3 cells of edge >= rc per axis:
 //               particles sorted by cell (the library's stable sort), one
-//               thread per target (in cell order) over the 27 neighbour cells.
+//               warp per target (in cell order) over the 27 neighbour cells.
 //               Each particle keeps its position wrapped into the box and the
 //               number of boxes it was moved by, so the image of a pair is
 //               recovered exactly and the reference's limit |p| <= layers on
 //               it holds for positions anywhere.
-// Scratch memory of the cell list is taken from the stream-ordered pool
-// (cudaMallocAsync) and returned on the same stream.
+// Scratch memory of the cell list is taken from a stream-ordered pool
+// (ScratchPool) and returned on the same stream.
 #include <cmath>
+#include <mutex>
 
 #include "se_internal.h"
 
@@ -134,54 +135,108 @@ __global__ void k_real_gather(RsParams S, const int* __restrict__ perm,
 
 __device__ __forceinline__ int kbox_of(int pk, int a) { return ((pk >> (10 * a)) & 1023) - 512; }
 
+// One warp per target (in cell order).  The lanes test 32 candidates of the
+// neighbour cells at a time -- a row of up to three z cells is one run of the
+// sorted particles -- and queue the pairs inside the cutoff; 32 queued pairs
+// are then evaluated together, one per lane.  About one candidate in eight is
+// a pair, and a pair costs some ten times a test (erfc, exp, two divisions):
+// with a target per thread most lanes of a warp sat out every evaluation
+// (50,000 particles, about 100 neighbours each, force: 548 -> 205 us; the FP64
+// pipe 35% and the issue slots 65% busy; with the separations queued instead
+// of the particles, 246 us).
+// A lane sums its pairs in queue order and the lanes' sums are added in a
+// fixed order, so results are deterministic.
 template <bool FORCE>
 __global__ void __launch_bounds__(RS_THREADS) k_real_cells(
     RsParams S, int nc, const double4* __restrict__ rec, const int* __restrict__ kbox,
-    const int* __restrict__ perm, const int* __restrict__ cell_off, const double* __restrict__ q,
-    double* __restrict__ phi, double* __restrict__ force)
+    const int* __restrict__ perm, const int* __restrict__ cell_off, double* __restrict__ phi,
+    double* __restrict__ force)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ int2 queue[RS_THREADS / 32][64];   // particle, box shifts + 1 (2 bits an axis)
+    const int s = blockIdx.x * (RS_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= S.N) return;
+    int2* que = queue[threadIdx.x >> 5];
     const double4 me = rec[s];
     const int km = kbox[s];
     const double xm[3] = {me.x, me.y, me.z};
     int c[3];
     for (int a = 0; a < 3; a++) c[a] = min((int)(xm[a] * nc / S.L), nc - 1);
+    // lane l < 18: run l, the z cells below or above the box's end (l odd) or
+    // the others of neighbour row l / 2, and its box shifts
+    int beg = 0, end = 0, shift = 0;
+    if (lane < 18) {
+        const int cx = c[0] + lane / 6 - 1, cy = c[1] + lane / 2 % 3 - 1;
+        const int sh0 = cx < 0 ? -1 : (cx >= nc ? 1 : 0);
+        const int sh1 = cy < 0 ? -1 : (cy >= nc ? 1 : 0);
+        const int row = ((cx - sh0 * nc) * nc + cy - sh1 * nc) * nc;
+        int z0 = max(c[2] - 1, 0), z1 = min(c[2] + 1, nc - 1);
+        int sh2 = 0;
+        if (lane & 1) {
+            sh2 = c[2] == 0 ? -1 : (c[2] == nc - 1 ? 1 : 0);
+            z0 = c[2] == 0 ? nc - 1 : 0;
+            z1 = sh2 ? z0 : z0 - 1;
+        }
+        beg = cell_off[row + z0];
+        end = cell_off[row + z1 + 1];
+        shift = (sh0 + 1) | (sh1 + 1) << 2 | (sh2 + 1) << 4;
+    }
     double acc = 0, f[3] = {0, 0, 0};
-    for (int dx = -1; dx <= 1; dx++)
-        for (int dy = -1; dy <= 1; dy++)
-            for (int dz = -1; dz <= 1; dz++) {
-                const int cc[3] = {c[0] + dx, c[1] + dy, c[2] + dz};
-                int w[3], sh[3];   // wrapped neighbour cell and its box shift
-                for (int a = 0; a < 3; a++) {
-                    sh[a] = cc[a] < 0 ? -1 : (cc[a] >= nc ? 1 : 0);
-                    w[a] = cc[a] - sh[a] * nc;
-                }
-                const int cell = (w[0] * nc + w[1]) * nc + w[2];
-                for (int t = cell_off[cell]; t < cell_off[cell + 1]; t++) {
-                    if (t == s && dx == 0 && dy == 0 && dz == 0) continue;
-                    const double4 o = rec[t];
-                    const double d[3] = {xm[0] - (o.x + sh[0] * S.L), xm[1] - (o.y + sh[1] * S.L),
-                                         xm[2] - (o.z + sh[2] * S.L)};
-                    const double rr = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-                    if (rr > S.rc2) continue;
-                    // the image index of the pair in raw coordinates
-                    const int kt = kbox[t];
-                    bool in = true;
-                    for (int a = 0; a < 3; a++) {
-                        const int p = kbox_of(kt, a) - kbox_of(km, a) - sh[a];
-                        in = in && p >= -S.layers && p <= S.layers;
-                    }
-                    if (in) pair_term<FORCE>(S, o.w, d, rr, acc, f);
-                }
+    auto separation = [&](const double4& o, int sh, double (&d)[3]) {
+        d[0] = xm[0] - (o.x + ((sh & 3) - 1) * S.L);
+        d[1] = xm[1] - (o.y + ((sh >> 2 & 3) - 1) * S.L);
+        d[2] = xm[2] - (o.z + ((sh >> 4 & 3) - 1) * S.L);
+        return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    };
+    auto pair = [&](int2 e) {
+        const double4 o = rec[e.x];
+        const int kt = kbox[e.x];
+        double d[3];
+        const double rr = separation(o, e.y, d);
+        bool in = true;   // the image index of the pair in raw coordinates
+        for (int a = 0; a < 3; a++) {
+            const int p = kbox_of(kt, a) - kbox_of(km, a) - ((e.y >> 2 * a & 3) - 1);
+            in = in && p >= -S.layers && p <= S.layers;
+        }
+        if (in) pair_term<FORCE>(S, o.w, d, rr, acc, f);
+    };
+    int queued = 0;
+    for (int run = 0; run < 18; run++) {
+        const int b = __shfl_sync(0xffffffffu, beg, run), e = __shfl_sync(0xffffffffu, end, run);
+        if (b >= e) continue;
+        const int sh = __shfl_sync(0xffffffffu, shift, run);
+        for (int t0 = b; t0 < e; t0 += 32) {
+            const int t = t0 + lane;
+            double d[3];
+            // (a particle is in one cell, so t = s is the pair with itself)
+            const bool in = t < e && t != s && !(separation(rec[min(t, e - 1)], sh, d) > S.rc2);
+            const unsigned hit = __ballot_sync(0xffffffffu, in);
+            if (in) que[queued + __popc(hit & ((1u << lane) - 1u))] = make_int2(t, sh);
+            queued += __popc(hit);
+            if (queued >= 32) {
+                __syncwarp();
+                pair(que[lane]);
+                queued -= 32;
+                const int2 rest = que[32 + lane];
+                __syncwarp();
+                if (lane < queued) que[lane] = rest;
             }
+        }
+    }
+    __syncwarp();
+    if (lane < queued) pair(que[lane]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (FORCE)
+            for (int a = 0; a < 3; a++) f[a] += __shfl_xor_sync(0xffffffffu, f[a], o);
+    }
+    if (lane != 0) return;
     const int m = perm[s];
     if (phi) phi[m] += acc;
     if (FORCE) {
-        const double qm = me.w;
-        force[m] += qm * f[0];
-        force[m + S.N] += qm * f[1];
-        force[m + 2 * S.N] += qm * f[2];
+        force[m] += me.w * f[0];
+        force[m + S.N] += me.w * f[1];
+        force[m + 2 * S.N] += me.w * f[2];
     }
 }
 
@@ -197,6 +252,52 @@ int cells_per_axis(double L, double rc)
     if (!(rc > 0) || 2 * rc > L) return 0;
     const double nc = floor(L / rc);
     return (nc >= 3 && nc <= 256) ? (int)nc : 0;
+}
+
+// Scratch of a call, ordered on its stream: from a pool of this library's own
+// that keeps up to KEEP bytes between calls (the device's default pool gives
+// everything back at the next synchronisation, and taking it again cost a call
+// that was waited for 0.5 ms); inside a stream capture from the default pool.
+struct ScratchPool {
+    static constexpr unsigned long long KEEP = 256ull << 20;
+    static constexpr int MAX_DEVICES = 64;
+    std::mutex mu;
+    cudaMemPool_t pool[MAX_DEVICES] = {};
+
+    int alloc(void** p, size_t bytes, cudaStream_t st)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        int dev = 0;
+        SE_CUDA(cudaGetDevice(&dev));
+        const bool plain = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+        if (!plain || dev >= MAX_DEVICES) {
+            cudaGetLastError();
+            SE_CUDA(cudaMallocAsync(p, bytes, st));
+            return SE_OK;
+        }
+        cudaMemPool_t mp;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!pool[dev]) {
+                cudaMemPoolProps props = {};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice;
+                props.location.id = dev;
+                SE_CUDA(cudaMemPoolCreate(&pool[dev], &props));
+                unsigned long long keep = KEEP;
+                SE_CUDA(cudaMemPoolSetAttribute(pool[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+            }
+            mp = pool[dev];
+        }
+        SE_CUDA(cudaMallocFromPoolAsync(p, bytes, mp, st));
+        return SE_OK;
+    }
+};
+
+ScratchPool& scratch_pool()
+{
+    static ScratchPool* p = new ScratchPool();
+    return *p;
 }
 
 int real_space(const double* x, const double* q, int N, double L, double xi, int layers,
@@ -225,7 +326,7 @@ int real_space(const double* x, const double* q, int N, double L, double xi, int
     const size_t obytes = 256 * ((sizeof(int) * (ncell + 1) + 255) / 256);
     const size_t total = 3 * nbytes + rbytes + obytes + sb;
     char* base = nullptr;
-    SE_CUDA(cudaMallocAsync((void**)&base, total, st));
+    SE_TRY(scratch_pool().alloc((void**)&base, total, st));
     int* key = reinterpret_cast<int*>(base);
     int* perm = reinterpret_cast<int*>(base + nbytes);
     int* kbox = reinterpret_cast<int*>(base + 2 * nbytes);
@@ -239,12 +340,9 @@ int real_space(const double* x, const double* q, int N, double L, double xi, int
         r = stable_sort(key, nullptr, N, ncell, perm, nullptr, off, scratch, sb, st, nullptr);
         if (r == SE_OK) {
             k_real_gather<<<ceil_div(N, 256), 256, 0, st>>>(S, perm, x, q, rec, kbox);
-            if (force)
-                k_real_cells<true><<<nb, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, q, phi,
-                                                              force);
-            else
-                k_real_cells<false><<<nb, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, q, phi,
-                                                               nullptr);
+            const unsigned nw = ceil_div(N, RS_THREADS / 32);
+            if (force) k_real_cells<true><<<nw, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, phi, force);
+            else k_real_cells<false><<<nw, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, phi, nullptr);
             e = cudaGetLastError();
         }
     }
