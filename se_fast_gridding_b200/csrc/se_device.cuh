@@ -24,6 +24,15 @@ __device__ __forceinline__ void f32x2_split(const float4& v, float2& lo, float2&
     hi = make_float2(v.z, v.w);
 }
 
+// D += A B on an 8 x 8 tile of FP64 sums, 4 deep: with g = lane / 4 and
+// t = lane % 4, a = A[g][t], b = B[t][g], d0 and d1 = D[g][2 t], D[g][2 t + 1].
+__device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+        : "+d"(d0), "+d"(d1)
+        : "d"(a), "d"(b));
+}
+
 // The tile-aligned kernels (k_spread2, k_interp2 on tile-aligned factor rows)
 // apply when a system's grid is cut into whole 16^3 tiles and its stencil
 // fits two tiles.
@@ -34,11 +43,32 @@ __host__ __device__ inline bool spread2_eligible(int M, int P)
 
 // A system's kernel path (SysDev::path): which spread and interpolation run.
 constexpr int PATH_TILE_SPREAD = 1;    // k_spread2 (else k_spread)
-constexpr int PATH_PAIR_INTERP = 2;    // k_interp2 (else k_interp / k_interp_global)
+constexpr int PATH_PAIR_INTERP = 2;    // k_interp2 or k_interp3 on tile-aligned rows
 constexpr int PATH_RUNTIME_P = 4;      // interpolation without the P-unrolled variants
 constexpr int PATH_RADIX_SORT = 8;     // the batch sorts with the radix passes (se_sort.cu)
 constexpr int PATH_FFT3 = 16;          // the batch's FP64 FFTs through se_fft.cuh (not cuFFT)
 constexpr int PATH_BIN_WINDOWS = 32;   // k_interp2 stages one window per bin (not per z pair)
+
+// Whether k_interp3 serves a system (else k_interp2 on the path with
+// PATH_PAIR_INTERP, k_interp without).  Measured on B200, interpolation stage:
+// - FP64 on tile-aligned rows: from M = 128 on, forces of P = 10 to 12 from M =
+//   192 on (M = 192, 1 to 80 particles per bin: 1.2 to 2.4x faster at P = 8 and
+//   16, potentials at P = 12 1.2 to 1.7x, forces at P = 12 0.96 to 1.1x); on
+//   smaller grids its warps are too few for their latency (M = 64: 0.7 to 1.1x);
+// - on other grids not for P <= 8 below M = 64 (M = 36, 1 to 18 per bin: 0.75
+//   to 1x, 4 us of a solve of 85);
+// - else FP64: always (M = 36 to 150, 1 to 120 per bin: 0.9 to 8x);
+// - else FP32: where the window kernel has no compiled-in stencil or,
+//   for potentials, gains nothing by it (P = 8 1.03 to 1.5x, P = 15 1.4 to 3x,
+//   P = 20 1.8 to 4.5x, potentials at P = 12 and 16 0.97 to 2x, forces there
+//   0.75 (120 per bin) to 1.5x (4 per bin)).
+__host__ __device__ inline bool interp3_better(int path, int precision, int M, int P, int mode)
+{
+    if (path & PATH_PAIR_INTERP)
+        return precision == SE_FP64 && M >= (mode == SE_FORCE && P >= 10 && P <= 12 ? 192 : 128);
+    if (P <= 8 && M < 64) return false;
+    return precision == SE_FP64 || mode == SE_POTENTIAL || (P != 12 && P != 16);
+}
 
 // The default path: the tile-aligned spread wherever it applies, and the
 // window-pair interpolation from P = 8 on (for shorter stencils its

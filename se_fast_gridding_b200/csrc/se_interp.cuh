@@ -2,6 +2,9 @@
 // SE_fgg.c:968-1100) with the periodic unfold (SE_FGG_extend_fcn,
 // SE_fgg.c:417-443) fused.  Included inside namespace se by se_solve.cu.
 //
+// k_interp: on grids that are not cut into whole tiles the FP32 forces of P =
+// 12 and 16 and the smallest systems of P <= 8 (elsewhere k_interp3 is faster:
+// interp3_better).
 // One CTA per fine bin (FB^3 stencil corners): the bin's window of
 // E = FB + P - 1 cells per axis is staged from the periodic grid into shared
 // memory (rows of the window are contiguous z runs of the grid; the periodic
@@ -69,18 +72,6 @@ __device__ __forceinline__ void set_factors(InterpWarpSmem<T>& W, const SysDev& 
     __syncwarp();
 }
 
-// The same from the factor array (lanes < P load their own entries).
-template <typename T>
-__device__ __forceinline__ void load_factors(InterpWarpSmem<T>& W, const SysDev& S,
-                                             const T* __restrict__ fac, int PS, long long p,
-                                             const double4& rc, int P, int lane)
-{
-    const T* f = fac + p * 3 * PS;
-    const bool in = lane < P;
-    set_factors(W, S, rc, P, lane, in ? f[lane] : T(0), in ? f[PS + lane] : T(0),
-                in ? f[2 * PS + lane] : T(0));
-}
-
 // PT = P at compile time (0: runtime P); plane = pitch between x planes of
 // the staged window (elements).
 template <typename T, int PT>
@@ -97,7 +88,7 @@ __global__ void __launch_bounds__(INTERP_WARPS * 32) k_interp(
     const int beg = boff[bin], end = boff[bin + 1];
     if (beg == end) return;
     const SysDev& S = sys[find_sys(bin_prefix, nsys, bin)];
-    if (S.path & PATH_PAIR_INTERP) return;   // k_interp2 covers this system
+    if ((S.path & PATH_PAIR_INTERP) || interp3_better(S.path, sizeof(T) == 4 ? SE_FP32 : SE_FP64, S.M, S.P, S.mode)) return;   // k_interp2, k_interp3
     const int P = PT ? PT : S.P;
     const int M = S.M;
     const int lb = bin - S.bin_base;
@@ -226,59 +217,4 @@ __global__ void __launch_bounds__(INTERP_WARPS * 32) k_interp(
                          phi_out);
         __syncwarp();
     }
-}
-
-// Interpolation without staging, for windows that exceed shared memory
-// (large P): the same sums read from the periodic grid through L1/L2.
-template <typename T>
-__global__ void __launch_bounds__(INTERP_WARPS * 32) k_interp_global(
-    const SysDev* __restrict__ sys, const int* __restrict__ part_prefix, int nsys, int ntot,
-    const double4* __restrict__ srec, const int* __restrict__ sg,
-    const int* __restrict__ sperm, const T* __restrict__ fac, int PS,
-    const T* __restrict__ rows, const double* __restrict__ grid, double* __restrict__ out,
-    double* __restrict__ phi_out)
-{
-    __shared__ InterpWarpSmem<T> wsm[INTERP_WARPS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int p = blockIdx.x * INTERP_WARPS + warp;
-    if (p >= ntot) return;
-    const int orig = sperm[p];
-    const SysDev& S = sys[find_sys(part_prefix, nsys, orig)];
-    if (S.path & PATH_PAIR_INTERP) return;   // k_interp2 covers this system
-    const int P = S.P, M = S.M;
-    InterpWarpSmem<T>& W = wsm[warp];
-    const double4 rc = srec[p];
-    const int pk = sg[p];
-    const int g0 = g_of(pk, 0), g1 = g_of(pk, 1), g2 = g_of(pk, 2);
-    load_factors(W, S, fac, PS, p, rc, P, lane);
-    const bool force = S.mode == SE_FORCE;
-    const double* gs = grid + S.grid_off;
-    double a_pot = 0, a_fx = 0, a_fy = 0, a_fz = 0;
-    for (int r = lane; r < P * P; r += 32) {
-        const int i = r / P, j = r % P;
-        const double* row = gs + ((long long)pmod(g0 + i, M) * M + pmod(g1 + j, M)) * M;
-        double s0 = 0, s1 = 0;
-        int z = g2;
-        for (int k = 0; k < P; k++) {
-            const double hv = __ldg(row + z);
-            s0 = fma(hv, (double)W.wz[k], s0);
-            if (force) s1 = fma(hv, (double)W.fz[k], s1);
-            if (++z == M) z = 0;
-        }
-        const double wxi = W.wx[i], wyj = W.wy[j];
-        a_pot = fma(s0, wxi * wyj, a_pot);
-        if (force) {
-            a_fx = fma(s0, W.fx[i] * wyj, a_fx);
-            a_fy = fma(s0, wxi * W.fy[j], a_fy);
-            a_fz = fma(s1, wxi * wyj, a_fz);
-        }
-    }
-    a_pot = warp_sum(a_pot);
-    if (force) {
-        a_fx = warp_sum(a_fx);
-        a_fy = warp_sum(a_fy);
-        a_fz = warp_sum(a_fz);
-    }
-    if (lane == 0)
-        interp_store(S, orig - S.part_off, rc.w, a_pot, a_fx, a_fy, a_fz, force, out, phi_out);
 }

@@ -1,0 +1,376 @@
+// se_interp3.cuh -- interpolation (SE_FGG_int / SE_FGG_int_force,
+// SE_fgg.c:968-1100) with the periodic unfold (SE_FGG_extend_fcn,
+// SE_fgg.c:417-443) fused, on FP64 matrix instructions, for any grid and
+// stencil.  Included inside namespace se by se_solve.cu after se_interp2.cuh.
+//
+// The particles of a fine bin (8^3 stencil corners) share a window of P + 7
+// grid cells per axis.  For a group of 8 of them the sum over y is a matrix
+// product: U[z][particle] = sum_y H[x][y][z] wy[y][particle], 8 z cells by 8
+// particles by 4 y per instruction, with the y weights zero outside each
+// stencil; forces take a second product with the y force weights.  U is
+// weighted with wx (and the force weights) and summed over the x planes in
+// the accumulators' own layout, then with wz.
+//
+// One CTA of 4 independent warps per bin (and per I3_PART further particles
+// of a crowded one); a warp takes a group at a time.  H comes straight from
+// the grid through L1: a window in shared memory (102 KB at P = 16, two CTAs
+// per SM) left the matrix unit idle while it was copied.  The operand tile is
+// laid so that its 8 rows are neighbouring z: a load touches 4 grid rows, and
+// two z tiles share 16-byte loads (the load wavefronts were the bound: 8 per
+// 8-byte load).  Forces load the next planes' operands into the registers of
+// the ones just used; potentials, with half the products per operand, do
+// better with more warps and no lookahead.
+//
+// The groups hold particles of neighbouring x offset, so they walk about P + 2
+// planes instead of P + 7.  A sum that is not finite is taken again over the
+// particle's own stencil: outside it the weights are zero, but zero times an
+// infinity of the caller's grid is not.
+//
+// B200, FP64, interpolation stage before (windows in shared memory, FP64
+// FMAs) and after: 100,000 particles, M = 128, P = 16 force 0.322 -> 0.257 ms,
+// potential 0.275 -> 0.190 ms; 20,000 particles, M = 100, P = 20, force 0.606
+// -> 0.139 ms; 2M clustered, M = 256, P = 12, force 3.34 -> 2.14 ms; 250,000,
+// M = 192, P = 12, potential 0.385 -> 0.305 ms; 1M, M = 256, P = 12, force 1.53
+// -> 1.55 ms, P = 8 potential 0.81 -> 0.49 ms.  At P = 16 the matrix unit is
+// 54% busy (its instructions alone take 0.126 ms), the load pipe 60%; the warps
+// in flight matter most (potentials with 4, 5 and 7 CTAs per SM at 250,000, P =
+// 12: 0.449, 0.315 and 0.305 ms; forces keep 128 registers, with fewer they
+// spill).
+
+constexpr int I3_WARPS = 4;
+constexpr int I3_PART = 256;   // particles of a bin a CTA takes
+// from this many particles on they are grouped by whether they reach the last
+// z tile (with fewer, groups of 8 stay partly empty: 30 per bin, P = 12, 1.61
+// -> 1.78 ms)
+constexpr int I3_BY_TILE = 64;
+
+// depth of the y contraction in steps of 4 cells over the window of a bin's
+// stencils, FB + P - 1 cells
+__host__ __device__ constexpr int interp3_nk(int P) { return (FB + P + 2) / 4; }
+
+// x planes a warp contracts together with nt z tiles (independent chains)
+__host__ __device__ constexpr int interp3_nx(bool force, int nt) { return force ? 2 / nt : 4 / nt; }
+
+// factor of cell w of a bin's window on axis a, for sorted particle p whose
+// stencil starts at cell r: from the tile-aligned rows, in which the window
+// starts at entry hw, or from the P-wide rows
+template <bool TILED, typename T>
+__device__ __forceinline__ double interp3_factor(const T* __restrict__ fac, int PS, int P, int p, int a, int w,
+                                                 int r, int hw)
+{
+    if constexpr (TILED) {
+        return (hw + w) < 32 ? (double)fac[(long long)p * 96 + 32 * a + hw + w] : 0.0;
+    } else {
+        const int i = w - r;
+        return (unsigned)i < (unsigned)P ? (double)fac[((long long)p * 3 + a) * PS + i] : 0.0;
+    }
+}
+
+// The same sum over particle p's own stencil alone, one cell after the other:
+// value q (potential, fx, fy, fz).
+template <bool TILED, typename T>
+__device__ __noinline__ double interp3_direct(const SysDev& S, const double* __restrict__ gs,
+                                              const T* __restrict__ fac, int PS, int p, int pk, double4 rc, int q)
+{
+    const int P = S.P, M = S.M;
+    auto weight = [&](int a, int i) -> double {
+        const double f = TILED ? (double)fac[(long long)p * 96 + 32 * a + (g_of(pk, a) & 15) + i]
+                               : (double)fac[((long long)p * 3 + a) * PS + i];
+        const double u = a == 0 ? rc.x : (a == 1 ? rc.y : rc.z);
+        return q == a + 1 ? f * (-S.c * (u - (S.lo + i) * S.h)) : f;
+    };
+    double sum = 0.0;
+    for (int i = 0; i < P; i++) {
+        double sx = 0.0;
+        for (int j = 0; j < P; j++) {
+            const double* row =
+                gs + ((long long)((g_of(pk, 0) + i) % M) * M + (g_of(pk, 1) + j) % M) * M;
+            double sy = 0.0;
+            for (int k = 0; k < P; k++) sy += row[(g_of(pk, 2) + k) % M] * weight(2, k);
+            sx += sy * weight(1, j);
+        }
+        sum += sx * weight(0, i);
+    }
+    return sum;
+}
+
+// SHARE (launches of few bins): the z tiles of one or two groups go over all
+// the warps
+template <int NK, bool FORCE, bool TILED, bool SHARE, typename T>
+__global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
+    const SysDev* __restrict__ sys, const int* __restrict__ part_prefix, int nsys, const int* __restrict__ tab,
+    int units, int P, const double4* __restrict__ srec, const int* __restrict__ sg,
+    const int* __restrict__ sperm, const T* __restrict__ fac, int PS,
+    const int* __restrict__ boff, const double* __restrict__ grid, double* __restrict__ out,
+    double* __restrict__ phi_out)
+{
+    constexpr int XE = 4 * NK + 2 * interp3_nx(FORCE, 1);
+    __shared__ unsigned char order[I3_PART];
+    __shared__ int start[2 * FB + 1];
+    __shared__ int xoff[XE];
+    __shared__ __align__(16) double wtab[I3_WARPS][FORCE ? 2 : 1][XE][8];   // the warps' x weights
+    // the tiles' sums of every lane of shared groups
+    __shared__ double part[SHARE ? 2 : 1][SHARE ? (NK + 1) / 2 : 1][FORCE ? 6 : 2][32];
+    // ---- the CTA's particles [c0, c0 + n) of one bin
+    const int unit = blockIdx.x;
+    int c0, n, sysi, bin;
+    if (unit < units) {   // the first of unit's bin
+        bin = __ldg(tab + units + unit);
+        sysi = __ldg(tab + unit);
+        c0 = boff[bin];
+        n = min(I3_PART, boff[bin + 1] - c0);
+    } else {   // of the sorted particles [s0, s0 + I3_PART) those past the
+               // first I3_PART of the bin that holds s0
+        const int s0 = (unit - units) * I3_PART;
+        sysi = find_sys(part_prefix, nsys, sperm[s0]);
+        const SysDev& S = sys[sysi];
+        if (S.P != P || S.mode != (FORCE ? SE_FORCE : SE_POTENTIAL) ||
+            ((S.path & PATH_PAIR_INTERP) != 0) != TILED)
+            return;
+        const int pk = sg[s0];
+        bin = S.bin_base + (g_of(pk, 0) / FB * S.nf[1] + g_of(pk, 1) / FB) * S.nf[2] + g_of(pk, 2) / FB;
+        c0 = max(boff[bin] + I3_PART, s0);
+        n = min(boff[bin + 1], s0 + I3_PART) - c0;
+    }
+    if (n <= 0) return;
+    const SysDev& S = sys[sysi];
+    const int lb = bin - S.bin_base, M = S.M;
+    const int o0 = (lb / (S.nf[1] * S.nf[2])) * FB, o1 = ((lb / S.nf[2]) % S.nf[1]) * FB,
+              o2 = (lb % S.nf[2]) * FB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const double* gs = grid + S.grid_off;
+    auto wrap = [&](int i) { return TILED ? (i >= M ? i - M : i) : i % M; };
+    for (int x = threadIdx.x; x < XE; x += blockDim.x) xoff[x] = wrap(o0 + x) * M * M;
+    int yoff[NK];
+#pragma unroll
+    for (int k = 0; k < NK; k++) yoff[k] = wrap(o1 + 4 * k + t) * M;
+    const double c = S.c, h = S.h;
+    const int hx = o0 & 8, hy = o1 & 8, hz = o2 & 8;
+    const int nz = (FB + P + 6) / 8;
+    double(*wx)[8] = wtab[warp][0], (*fx)[8] = wtab[warp][FORCE ? 1 : 0];
+
+    // ---- the particles ordered by whether their stencil reaches the last z
+    // tile and by x offset: the groups of 8 then span few x and often leave
+    // that tile out (any order does: a particle's sums do not depend on its
+    // group)
+    const bool by_tile = n >= I3_BY_TILE && 8 * (nz - 1) - P >= 2;
+    auto rank = [&](int i) {
+        const int pk = sg[c0 + i];
+        return (by_tile && g_of(pk, 2) - o2 + P > 8 * (nz - 1) ? FB : 0) + g_of(pk, 0) - o0;
+    };
+    if (n > 8) {
+        if (threadIdx.x <= 2 * FB) start[threadIdx.x] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&start[rank(i) + 1], 1);
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 1; i < 2 * FB; i++) start[i] += start[i - 1];
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) order[atomicAdd(&start[rank(i)], 1)] = (unsigned char)i;
+    } else if (threadIdx.x < n) {
+        order[threadIdx.x] = threadIdx.x;
+    }
+    __syncthreads();
+    {
+        const int share = !SHARE ? 1 : (n <= 8 ? I3_WARPS : (n <= 16 ? I3_WARPS / 2 : 1));
+        for (int g0 = 8 * (warp / share); g0 < n; g0 += 8 * I3_WARPS / share) {
+            // ---- the group's weights.  Lane (g, t): y weights of particle g
+            // at y = 4 k + t; x weights in shared memory; z weights of
+            // particles 2 t, 2 t + 1 at z = 8 i + g (below)
+            const bool valid = g0 + g < n;
+            const int p = c0 + order[min(g0 + g, n - 1)];
+            const int pk = sg[p];
+            const double4 rc = srec[p];
+            const int rx = g_of(pk, 0) - o0, ry = g_of(pk, 1) - o1, rz = g_of(pk, 2) - o2;
+            double by[NK], fy[FORCE ? NK : 1];
+            const double uy = rc.y - (S.lo - ry) * h;
+#pragma unroll
+            for (int k = 0; k < NK; k++) {
+                by[k] = valid ? interp3_factor<TILED>(fac, PS, P, p, 1, 4 * k + t, ry, hy) : 0.0;
+                if (FORCE) fy[k] = by[k] * (-c * (uy - (4 * k + t) * h));
+            }
+            int xlo = rx, xhi = rx + P;
+            {
+                const int src = (lane & 7) * 4;
+                const int pn = __shfl_sync(0xffffffffu, p, src);
+                const int rn = __shfl_sync(0xffffffffu, rx, src);
+                const double ux = __shfl_sync(0xffffffffu, rc.x, src) - (S.lo - rn) * h;
+                for (int x = lane >> 3; x < XE; x += 4) {
+                    const double w = x < 4 * NK ? interp3_factor<TILED>(fac, PS, P, pn, 0, x, rn, hx) : 0.0;
+                    wx[x][lane & 7] = w;
+                    if (FORCE) fx[x][lane & 7] = w * (-c * (ux - x * h));
+                }
+                xlo = __reduce_min_sync(0xffffffffu, xlo);
+                xhi = __reduce_max_sync(0xffffffffu, xhi);
+            }
+            int pz[2], rzn[2];
+            double uz[2];
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const int src = (2 * t + b) * 4;
+                pz[b] = __shfl_sync(0xffffffffu, p, src);
+                rzn[b] = __shfl_sync(0xffffffffu, rz, src);
+                uz[b] = __shfl_sync(0xffffffffu, rc.z, src) - (S.lo - rzn[b]) * h;
+            }
+            __syncwarp();
+            const int ztop = __reduce_max_sync(0xffffffffu, rz) + P;
+            double s[2][4] = {};
+            // the sums over x at the lane's cell z of a tile, with the z weights
+            auto add_tile = [&](int z, const double (&ap)[2], const double (&ax)[2], const double (&ay)[2]) {
+#pragma unroll
+                for (int b = 0; b < 2; b++) {
+                    const double wz = interp3_factor<TILED>(fac, PS, P, pz[b], 2, z, rzn[b], hz);
+                    s[b][0] = fma(wz, ap[b], s[b][0]);
+                    if (FORCE) {
+                        s[b][1] = fma(wz, ax[b], s[b][1]);
+                        s[b][2] = fma(wz, ay[b], s[b][2]);
+                        s[b][3] = fma(wz * (-c * (uz[b] - z * h)), ap[b], s[b][3]);
+                    }
+                }
+            };
+            // U[z][particle] = sum_y H[x][y][z] wy of NX planes x and NT z
+            // tiles, then the sums over x with the x weights.  Two tiles
+            // share 16-byte loads: the rows of the first are the even z of
+            // their 16, those of the second the odd ones
+            auto tiles = [&](int i, auto nt) {
+                constexpr int NT = decltype(nt)::value, NX = interp3_nx(FORCE, NT);
+                const double* col = gs + wrap(o2 + 8 * i + NT * g);
+                double ap[NT][2] = {}, ax[NT][2] = {}, ay[NT][2] = {};
+                double a[NX][NK][NT];
+                auto load = [&](int x, int j, int k) {
+                    const double* cell = col + xoff[x + j] + yoff[k];
+                    if constexpr (NT == 2) {
+                        const double2 w = __ldg(reinterpret_cast<const double2*>(cell));
+                        a[j][k][0] = w.x;
+                        a[j][k][1] = w.y;
+                    } else {
+                        a[j][k][0] = __ldg(cell);
+                    }
+                };
+                auto load_all = [&](int x) {
+#pragma unroll
+                    for (int k = 0; k < NK; k++)
+#pragma unroll
+                        for (int j = 0; j < NX; j++) load(x, j, k);
+                };
+                if (FORCE) load_all(xlo);
+#pragma unroll 1
+                for (int x = xlo; x < xhi; x += NX) {
+                    if (!FORCE) load_all(x);
+                    double u[NX][NT][2] = {}, v[FORCE ? NX : 1][NT][2] = {};
+#pragma unroll
+                    for (int k = 0; k < NK; k++) {
+#pragma unroll
+                        for (int j = 0; j < NX; j++) {
+#pragma unroll
+                            for (int m = 0; m < NT; m++) {
+                                mma_f64(u[j][m][0], u[j][m][1], a[j][k][m], by[k]);
+                                if (FORCE) mma_f64(v[j][m][0], v[j][m][1], a[j][k][m], fy[k]);
+                            }
+                        }
+                        // the operands of the next planes take their place
+                        // (past the window: read, not used)
+                        if (FORCE) {
+#pragma unroll
+                            for (int j = 0; j < NX; j++) load(x + NX, j, k);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < NX; j++) {
+                        const double2 w = *reinterpret_cast<const double2*>(&wx[x + j][2 * t]);
+                        double2 f = make_double2(0.0, 0.0);
+                        if (FORCE) f = *reinterpret_cast<const double2*>(&fx[x + j][2 * t]);
+#pragma unroll
+                        for (int m = 0; m < NT; m++) {
+                            ap[m][0] = fma(w.x, u[j][m][0], ap[m][0]);
+                            ap[m][1] = fma(w.y, u[j][m][1], ap[m][1]);
+                            if (FORCE) {
+                                ax[m][0] = fma(f.x, u[j][m][0], ax[m][0]);
+                                ax[m][1] = fma(f.y, u[j][m][1], ax[m][1]);
+                                ay[m][0] = fma(w.x, v[j][m][0], ay[m][0]);
+                                ay[m][1] = fma(w.y, v[j][m][1], ay[m][1]);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < NT; m++) {
+                    if (share == 1) {
+                        add_tile(8 * i + NT * g + m, ap[m], ax[m], ay[m]);
+                        continue;
+                    }
+                    double(*pt)[32] = part[SHARE ? g0 / 8 : 0][SHARE ? i + m : 0];
+                    pt[0][lane] = ap[m][0];
+                    pt[1][lane] = ap[m][1];
+                    if (FORCE) {
+                        pt[2][lane] = ax[m][0];
+                        pt[3][lane] = ax[m][1];
+                        pt[4][lane] = ay[m][0];
+                        pt[5][lane] = ay[m][1];
+                    }
+                }
+            };
+            // the tiles two at a time where rows are 16-byte aligned and do
+            // not wrap inside a pair of cells (even M), the last of an odd
+            // number alone; those that no stencil of the group reaches add
+            // nothing and are left out
+            const int pairs = M % 2 == 0 ? nz / 2 : 0;
+            for (int i = warp % share; i < nz - pairs; i += share) {
+                if (i < pairs) {
+                    if (16 * i < ztop) tiles(2 * i, std::integral_constant<int, 2>());
+                } else if (8 * (pairs + i) < ztop) {
+                    tiles(pairs + i, std::integral_constant<int, 1>());
+                }
+            }
+            if (share > 1) {   // the group's first warp adds the tiles, in order
+                __syncthreads();   // (one round: every warp gets here once)
+                if (warp % share != 0) continue;
+                for (int i = 0; i < nz; i++) {
+                    const bool paired = i < 2 * pairs;
+                    if (8 * (paired ? i & ~1 : i) >= ztop) break;
+                    const double(*pt)[32] = part[SHARE ? g0 / 8 : 0][SHARE ? i : 0];
+                    const double ap[2] = {pt[0][lane], pt[1][lane]};
+                    double ax[2] = {0, 0}, ay[2] = {0, 0};
+                    if (FORCE) {
+                        ax[0] = pt[2][lane];
+                        ax[1] = pt[3][lane];
+                        ay[0] = pt[4][lane];
+                        ay[1] = pt[5][lane];
+                    }
+                    add_tile(paired ? 16 * (i / 2) + 2 * g + i % 2 : 8 * i + g, ap, ax, ay);
+                }
+            }
+            // ---- the sums over the 8 lanes of each particle pair, by halving:
+            // lane (g, t) ends with value g & 3 (potential, fx, fy, fz) of
+            // particle 2 t + (g >> 2)
+            const bool g2 = g & 4, g1 = g & 2, g0b = g & 1;
+            double r[4];
+#pragma unroll
+            for (int q = 0; q < (FORCE ? 4 : 1); q++)
+                r[q] = (g2 ? s[1][q] : s[0][q]) + __shfl_xor_sync(0xffffffffu, g2 ? s[0][q] : s[1][q], 16);
+            double val;
+            if (FORCE) {
+                const double m0 = (g1 ? r[2] : r[0]) + __shfl_xor_sync(0xffffffffu, g1 ? r[0] : r[2], 8);
+                const double m1 = (g1 ? r[3] : r[1]) + __shfl_xor_sync(0xffffffffu, g1 ? r[1] : r[3], 8);
+                val = (g0b ? m1 : m0) + __shfl_xor_sync(0xffffffffu, g0b ? m0 : m1, 4);
+            } else {
+                val = r[0] + __shfl_xor_sync(0xffffffffu, r[0], 8);
+                val += __shfl_xor_sync(0xffffffffu, val, 4);
+            }
+            const int ip = 2 * t + (g >> 2), q = FORCE ? g & 3 : 0;
+            if (g0 + ip < n && (FORCE || (g & 3) == 0)) {
+                const int pm = c0 + order[g0 + ip];
+                const int loc = sperm[pm] - S.part_off;
+                const double scale = S.h3 * S.d;
+                if (!isfinite(val)) val = interp3_direct<TILED>(S, gs, fac, PS, pm, sg[pm], srec[pm], q);
+                if (q == 0) {
+                    double* dst = FORCE ? phi_out : out;
+                    if (dst) dst[(FORCE ? S.part_off : S.out_off) + loc] = scale * val;
+                } else {
+                    out[S.out_off + loc + (long long)(q - 1) * S.N] = srec[pm].w / S.d * scale * val;
+                }
+            }
+            __syncwarp();   // the x weights are read before the next group's
+        }
+    }
+}

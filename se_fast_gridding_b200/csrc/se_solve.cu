@@ -17,10 +17,10 @@
 //               P <= 16; k_spread (se_spread.cuh) for the others
 //   cuFFT D2Z, k_scale (Z of scaling(), SE_general.c:145-175, applied to the
 //               half spectrum as product_rc does, SE_general.c:336-362), Z2D
-//   interp      k_grid_to_f32 (FP32 path) + k_interp2, one launch per stencil
-//               of the batch, one CTA per fine bin or pair of z-adjacent bins
-//               of its systems, the unfold fused (se_interp2.cuh), beside
-//               k_spread2; k_interp (se_interp.cuh) for the others
+//   interp      one launch per stencil and mode of the batch, the unfold fused:
+//               k_interp3 (se_interp3.cuh; FP64 on larger grids, most others),
+//               k_interp2 (se_interp2.cuh; in FP32 from k_grid_to_f32's copy)
+//               beside k_spread2, k_interp (se_interp.cuh) for the rest
 //
 // Grid layout: M^3 FP64 row-major [x][y][z], the transpose of the reference's
 // column-major H_per; the FFT of the transpose is the transpose of the FFT and
@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(SCALE_THREADS) k_scale32(const SysDev* __restr
 #include "se_fft.cuh"
 #include "se_interp.cuh"
 #include "se_interp2.cuh"
+#include "se_interp3.cuh"
 
 // FP32 grid back to FP64 (the FP32-FFT path feeding the general interpolation
 // or a caller's FP64 grid).
@@ -419,7 +420,7 @@ struct se_batch_s {
     // S2_BLOCKS_MANY
     bool spread2_few = false;
     bool any_spread1 = false, any_spread2 = false;   // some system on k_spread / k_spread2
-    bool any_interp1 = false, any_interp2 = false;   // on k_interp(_global) / k_interp2
+    bool any_interp1 = false, any_interp2 = false;   // on k_interp / with PATH_PAIR_INTERP
     bool runtime_p = false;                          // some system asks for runtime P
     float* grid32 = nullptr;  // FP32 copy of the grids, staged by k_interp2<float>
     bool fft32 = false;       // SE_FP32_FFT32: FP32 FFTs on grid32 / spec32
@@ -434,6 +435,9 @@ struct se_batch_s {
         int Ep = 0, PL = 0;     // window pitches
         int zb = 1;             // z-adjacent bins per window (1 or 2)
         size_t smem = 0;
+        bool mma = false;       // k_interp3
+        bool tiled = false;     // from tile-aligned factor rows
+        int mode = SE_POTENTIAL;
         int units = 0;          // CTAs: the systems' bins / zb
         int* tab = nullptr;     // device: each unit's system, then its first bin
     };
@@ -451,7 +455,7 @@ struct se_batch_s {
     int launches = 0;
     int pending_launches = 0;   // issued before the next solve's own launches (rebind)
     int max_P = 0;
-    bool staged_interp = true;
+    int interp_P = 0;        // the stencil of the k_interp systems (0: several)
     size_t interp_smem = 0;
     int plane = 0;   // x-plane pitch of the staged interpolation window
     // per-stage CUDA events (prepare+sort, spread, k-space, interp)
@@ -545,8 +549,7 @@ static int interp_plane(int P)
 
 static size_t interp_smem_bytes(int P, int precision)
 {
-    const int E = FB + P - 1;
-    return (size_t)E * interp_plane(P) * (precision == SE_FP32 ? 4 : 8);
+    return (precision == SE_FP32 ? 4 : 8) * (size_t)(FB + P - 1) * interp_plane(P);
 }
 
 static int path_of(const se_system* sys, const int* paths, int i)
@@ -643,30 +646,16 @@ static int batch_free(se_batch b)
     return SE_OK;
 }
 
-// The staged interpolation kernel a batch launches: specialised on P when
-// every system has the same P in {8, 12, 16} (or 21 in FP64), else generic.
+// The k_interp kernel of a batch: specialised on P when all its systems have
+// the same and none asks for the runtime-P variants.
 template <typename T>
-static const void* staged_interp_variant(int P, bool uniform)
+static const void* interp_kernel(const se_batch_s* b)
 {
-    if (uniform && P == 8) return (const void*)k_interp<T, 8>;
-    if (uniform && P == 12) return (const void*)k_interp<T, 12>;
-    if (uniform && P == 16) return (const void*)k_interp<T, 16>;
-    if (sizeof(T) == 8 && uniform && P == 21) return (const void*)k_interp<T, 21>;
-    return (const void*)k_interp<T, 0>;
-}
-
-static bool uniform_P(const se_batch_s* b)
-{
-    if (b->runtime_p) return false;   // the runtime-P variants were asked for
-    for (auto& s : b->host_sys)
-        if (s.P != b->max_P) return false;
-    return true;
-}
-
-static const void* staged_interp_kernel(const se_batch_s* b)
-{
-    return b->precision == SE_FP32 ? staged_interp_variant<float>(b->max_P, uniform_P(b))
-                                   : staged_interp_variant<double>(b->max_P, uniform_P(b));
+    const int P = b->runtime_p ? 0 : b->interp_P;
+    return P == 8    ? (const void*)k_interp<T, 8>
+           : P == 12 ? (const void*)k_interp<T, 12>
+           : P == 16 ? (const void*)k_interp<T, 16>
+                     : (const void*)k_interp<T, 0>;
 }
 
 // Dynamic shared memory a kernel may use is a per-device, per-function
@@ -838,45 +827,44 @@ static int interp2_table(se_batch_s* b, se_batch_s::I2Class& c, const std::vecto
 // The k_interp2 launches of a batch (se_batch_s::i2_cls).
 static int interp2_classes(se_batch_s* b, const se_system* systems, int nsys)
 {
-    std::map<int, std::pair<long long, long long>> byP;   // P -> (particles, bins)
+    // the systems of one launch: one stencil and mode each; those of
+    // k_interp2 in one launch when some system asks for runtime P
+    struct Group {
+        long long particles = 0, bins = 0;
+        std::vector<int> members;
+    };
+    std::map<std::tuple<bool, bool, int, int>, Group> groups;   // (k_interp3, tiled, P, mode)
     bool bin_windows = false;
     int maxP = 0;
-    long long np = 0, nb = 0;
     for (int i = 0; i < nsys; i++) {
         const SysDev& S = b->host_sys[i];
-        if (!(S.path & PATH_PAIR_INTERP)) continue;
-        const long long bins = (long long)S.nf[0] * S.nf[1] * S.nf[2];
-        byP[systems[i].P].first += systems[i].N;
-        byP[systems[i].P].second += bins;
-        np += systems[i].N;
-        nb += bins;
-        maxP = std::max(maxP, systems[i].P);
-        if (S.mode == SE_FORCE) b->i2_force = true;
+        const bool mma = interp3_better(S.path, b->precision, S.M, S.P, S.mode), tiled = S.path & PATH_PAIR_INTERP;
+        if (!mma && !tiled) continue;
+        const bool any_p = b->runtime_p && !mma;
+        Group& g = groups[{mma, tiled, any_p ? 0 : S.P, any_p ? 0 : S.mode}];
+        g.particles += S.N;
+        g.bins += (long long)S.nf[0] * S.nf[1] * S.nf[2];
+        g.members.push_back(i);
+        if (!mma) maxP = std::max(maxP, S.P);
+        if (!mma && S.mode == SE_FORCE) b->i2_force = true;
         if (S.path & PATH_BIN_WINDOWS) bin_windows = true;
     }
     b->i2_cls.clear();
-    auto members = [&](int P) {   // the pair-interpolation systems of stencil P (0: all)
-        std::vector<int> v;
-        for (int i = 0; i < nsys; i++)
-            if ((b->host_sys[i].path & PATH_PAIR_INTERP) && (P == 0 || systems[i].P == P))
-                v.push_back(i);
-        return v;
-    };
-    if (b->runtime_p) {
+    for (const auto& kv : groups) {
         b->i2_cls.emplace_back();
         se_batch_s::I2Class& c = b->i2_cls.back();
-        c.P = 0;
-        c.Pw = maxP;
-        SE_TRY(interp2_window(b, c, np, nb, bin_windows));
-        return interp2_table(b, c, members(0));
-    }
-    for (const auto& kv : byP) {
-        b->i2_cls.emplace_back();
-        se_batch_s::I2Class& c = b->i2_cls.back();
-        c.P = c.Pw = kv.first;
-        c.special = interp2_special(kv.first);
-        SE_TRY(interp2_window(b, c, kv.second.first, kv.second.second, bin_windows));
-        SE_TRY(interp2_table(b, c, members(kv.first)));
+        c.mma = std::get<0>(kv.first);
+        c.tiled = std::get<1>(kv.first);
+        c.P = std::get<2>(kv.first);
+        c.mode = std::get<3>(kv.first);
+        c.Pw = c.P ? c.P : maxP;
+        if (c.mma) {
+            c.zb = 1;
+        } else {
+            c.special = c.P && interp2_special(c.P);
+            SE_TRY(interp2_window(b, c, kv.second.particles, kv.second.bins, bin_windows));
+        }
+        SE_TRY(interp2_table(b, c, kv.second.members));
     }
     return SE_OK;
 }
@@ -968,9 +956,6 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
             b->spread2_few = b->ntiles <= S2_BLOCKS_FEW * sms;
     }
-    b->interp_smem = interp_smem_bytes(b->max_P, precision);
-    b->plane = interp_plane(b->max_P);
-    b->staged_interp = b->interp_smem + sizeof(InterpWarpSmem<double>) * INTERP_WARPS <= 220 * 1024;
 
     auto fail = [&](int code) {
         batch_free(b);
@@ -995,10 +980,16 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
     SE_ALLOC(b->boff, sizeof(int) * (b->nbins + 1));
     b->PS = b->max_P;
     bool need_fac = false, need_rows = false;
+    int window_P = 0;   // the largest stencil of the k_interp systems
     for (int i = 0; i < nsys; i++) {
         const int path = b->host_sys[i].path;
         (path & PATH_TILE_SPREAD ? b->any_spread2 : b->any_spread1) = true;
-        (path & PATH_PAIR_INTERP ? b->any_interp2 : b->any_interp1) = true;
+        if (path & PATH_PAIR_INTERP) b->any_interp2 = true;
+        else if (const SysDev& S = b->host_sys[i]; !interp3_better(path, precision, S.M, S.P, S.mode)) {
+            b->interp_P = !b->any_interp1 || b->interp_P == S.P ? S.P : 0;
+            window_P = std::max(window_P, S.P);
+            b->any_interp1 = true;
+        }
         if (path & PATH_RUNTIME_P) b->runtime_p = true;
         const int t = path & (PATH_TILE_SPREAD | PATH_PAIR_INTERP);
         if (t) need_rows = true;
@@ -1025,7 +1016,7 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
     if ((b->any_interp2 && precision == SE_FP32) || fft32)
         SE_ALLOC(b->grid32, sizeof(float) * (b->grid_elems + 16));
     if (fft32) SE_ALLOC(b->spec32, sizeof(float2) * b->spec_elems);
-    if (b->any_interp2) {
+    {
         const int rc = interp2_classes(b, systems, nsys);
         if (rc != SE_OK) return fail(rc);
     }
@@ -1114,8 +1105,11 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
                                      cudaFuncAttributePreferredSharedMemoryCarveout, carve);
         if (a != cudaSuccess) return fail(cuda_fail(a, "cudaFuncSetAttribute", __FILE__, __LINE__));
     }
-    if (b->staged_interp) {
-        const cudaError_t a = raise_smem_limit(staged_interp_kernel(b), b->interp_smem);
+    if (b->any_interp1) {
+        b->interp_smem = interp_smem_bytes(window_P, precision);
+        b->plane = interp_plane(window_P);
+        const cudaError_t a = raise_smem_limit(
+            precision == SE_FP32 ? interp_kernel<float>(b) : interp_kernel<double>(b), b->interp_smem);
         if (a != cudaSuccess) return fail(cuda_fail(a, "cudaFuncSetAttribute", __FILE__, __LINE__));
     }
     for (const auto& g : b->groups) {
@@ -1328,23 +1322,12 @@ static int run_kspace(se_batch b, double* grid, cudaStream_t st, bool* grid32_fr
 }
 
 template <typename T>
-static int launch_interp_staged(se_batch b, const double* grid, double* out, double* phi,
-                                cudaStream_t st)
+static int launch_interp(se_batch b, const double* grid, double* out, double* phi, cudaStream_t st)
 {
-    const size_t smem = b->interp_smem;
-    const int P = b->max_P;
-    const bool uniform = uniform_P(b);
-    const dim3 grd(std::max(b->nbins, 1)), blk(INTERP_WARPS * 32);
-    const T* fac = static_cast<const T*>(b->fac);
-    const T* rows = static_cast<const T*>(b->rows);
-#define SE_IARGS b->sys, b->d_bin_prefix, b->nsys, b->srec, b->sg, b->perm, fac, b->PS, rows, \
-                 b->boff, grid, out, phi, b->plane
-    if (uniform && P == 8) k_interp<T, 8><<<grd, blk, smem, st>>>(SE_IARGS);
-    else if (uniform && P == 12) k_interp<T, 12><<<grd, blk, smem, st>>>(SE_IARGS);
-    else if (uniform && P == 16) k_interp<T, 16><<<grd, blk, smem, st>>>(SE_IARGS);
-    else if (sizeof(T) == 8 && uniform && P == 21) k_interp<T, 21><<<grd, blk, smem, st>>>(SE_IARGS);
-    else k_interp<T, 0><<<grd, blk, smem, st>>>(SE_IARGS);
-#undef SE_IARGS
+    const auto fn = reinterpret_cast<decltype(&k_interp<T, 0>)>(interp_kernel<T>(b));
+    fn<<<std::max(b->nbins, 1), INTERP_WARPS * 32, b->interp_smem, st>>>(
+        b->sys, b->d_bin_prefix, b->nsys, b->srec, b->sg, b->perm, static_cast<const T*>(b->fac), b->PS,
+        static_cast<const T*>(b->rows), b->boff, grid, out, phi, b->plane);
     SE_CUDA(cudaGetLastError());
     LAUNCHED(b);
     return SE_OK;
@@ -1376,7 +1359,7 @@ static int launch_interp2_mode(se_batch b, const T* grid, double* out, double* p
     const dim3 blk(I2_WARPS * 32);
     const T* rows = static_cast<const T*>(b->rows);
     for (const auto& c : b->i2_cls) {
-        if (c.units == 0) continue;
+        if (c.units == 0 || c.mma) continue;
         const dim3 grd(c.units);
         const void* fn = interp2_kernel<T, FORCE>(c.Pw, c.special);
         SE_CUDA(raise_smem_limit(fn, c.smem));
@@ -1401,6 +1384,50 @@ static int launch_interp2(se_batch b, const T* grid, double* out, double* phi, c
                      : launch_interp2_mode<T, false>(b, grid, out, phi, st);
 }
 
+// Launches of at most this many bins (about four CTAs per SM) share a bin's z
+// tiles among the warps: 100 particles, M = 32, P = 21 27 -> 16 us with it; on
+// larger grids the repeated weights cost more than the idle warps.  The sums
+// are the same either way.
+constexpr int I3_SHARE_UNITS = 600;
+
+template <int NK, typename T>
+static int launch_interp3(se_batch b, const se_batch_s::I2Class& c, const double* grid, double* out,
+                          double* phi, cudaStream_t st)
+{
+    const bool force = c.mode == SE_FORCE;
+    const bool share = c.units <= I3_SHARE_UNITS;
+    auto fn = share ? (force ? k_interp3<NK, true, false, true, T> : k_interp3<NK, false, false, true, T>)
+                    : (force ? k_interp3<NK, true, false, false, T> : k_interp3<NK, false, false, false, T>);
+    if constexpr (NK <= interp3_nk(16) && sizeof(T) == 8)   // tile-aligned rows: FP64, P <= 16, larger grids
+        if (c.tiled) fn = force ? k_interp3<NK, true, true, false, T> : k_interp3<NK, false, true, false, T>;
+    fn<<<c.units + ceil_div(b->ntot, I3_PART), I3_WARPS * 32, 0, st>>>(
+        b->sys, b->d_part_prefix, b->nsys, c.tab, c.units, c.P, b->srec, b->sg, b->perm,
+        static_cast<const T*>(c.tiled ? b->rows : b->fac), b->PS, b->boff, grid, out, phi);
+    SE_CUDA(cudaGetLastError());
+    LAUNCHED(b);
+    return SE_OK;
+}
+
+template <typename T>
+static int run_interp3(se_batch b, const double* grid, double* out, double* phi, cudaStream_t st)
+{
+    for (const auto& c : b->i2_cls) {
+        if (!c.mma || c.units == 0) continue;
+        switch (interp3_nk(c.P)) {
+        case 2: SE_TRY((launch_interp3<2, T>(b, c, grid, out, phi, st))); break;
+        case 3: SE_TRY((launch_interp3<3, T>(b, c, grid, out, phi, st))); break;
+        case 4: SE_TRY((launch_interp3<4, T>(b, c, grid, out, phi, st))); break;
+        case 5: SE_TRY((launch_interp3<5, T>(b, c, grid, out, phi, st))); break;
+        case 6: SE_TRY((launch_interp3<6, T>(b, c, grid, out, phi, st))); break;
+        case 7: SE_TRY((launch_interp3<7, T>(b, c, grid, out, phi, st))); break;
+        case 8: SE_TRY((launch_interp3<8, T>(b, c, grid, out, phi, st))); break;
+        case 9: SE_TRY((launch_interp3<9, T>(b, c, grid, out, phi, st))); break;
+        default: SE_TRY((launch_interp3<10, T>(b, c, grid, out, phi, st))); break;
+        }
+    }
+    return SE_OK;
+}
+
 // grid32_fresh: grid32 holds the FP32 copy of `grid` already.
 // grid32_ready: the FP32-FFT k-space step left the grids in grid32 (the FP64
 // `grid` is then rebuilt from it only for the general interpolation).
@@ -1408,35 +1435,25 @@ static int run_interp(se_batch b, double* grid, double* out, double* phi, cudaSt
                       bool grid32_ready = false, bool grid32_fresh = false)
 {
     if (b->ntot == 0) return SE_OK;
-    // systems of whole 16^3 tiles with P <= 16: k_interp2 (FP32 path from an
-    // FP32 copy of the grids); the others: k_interp / k_interp_global
-    if (b->any_interp2) {
-        if (b->precision == SE_FP32) {
+    // (interp3_better says which kernel serves a system)
+    bool pairs = false, mma = false;   // some system on k_interp2, on k_interp3
+    for (const auto& c : b->i2_cls) (c.mma ? mma : pairs) |= c.units > 0;
+    if ((mma || b->any_interp1) && grid32_ready) SE_TRY(grid_f32_to_f64(b, grid, st));
+    if (mma) {
+        if (b->precision == SE_FP64) SE_TRY(run_interp3<double>(b, grid, out, phi, st));
+        else SE_TRY(run_interp3<float>(b, grid, out, phi, st));
+    }
+    if (pairs) {
+        if (b->precision == SE_FP64) {
+            SE_TRY(launch_interp2<double>(b, grid, out, phi, st));
+        } else {
             if (!grid32_ready && !grid32_fresh) SE_TRY(grid_f64_to_f32(b, grid, st));
             SE_TRY(launch_interp2<float>(b, b->grid32, out, phi, st));
-        } else {
-            SE_TRY(launch_interp2<double>(b, grid, out, phi, st));
         }
     }
-    if (!b->any_interp1) return SE_OK;
-    if (grid32_ready) SE_TRY(grid_f32_to_f64(b, grid, st));
-    if (b->staged_interp) {
-        if (b->precision == SE_FP32) return launch_interp_staged<float>(b, grid, out, phi, st);
-        return launch_interp_staged<double>(b, grid, out, phi, st);
-    }
-    const unsigned nb = ceil_div(b->ntot, INTERP_WARPS);
-    if (b->precision == SE_FP32)
-        k_interp_global<float><<<nb, INTERP_WARPS * 32, 0, st>>>(
-            b->sys, b->d_part_prefix, b->nsys, b->ntot, b->srec, b->sg, b->perm,
-            static_cast<const float*>(b->fac), b->PS, static_cast<const float*>(b->rows), grid,
-            out, phi);
-    else
-        k_interp_global<double><<<nb, INTERP_WARPS * 32, 0, st>>>(
-            b->sys, b->d_part_prefix, b->nsys, b->ntot, b->srec, b->sg, b->perm,
-            static_cast<const double*>(b->fac), b->PS, static_cast<const double*>(b->rows), grid,
-            out, phi);
-    SE_CUDA(cudaGetLastError());
-    LAUNCHED(b);
+    if (b->any_interp1)
+        SE_TRY(b->precision == SE_FP64 ? launch_interp<double>(b, grid, out, phi, st)
+                                       : launch_interp<float>(b, grid, out, phi, st));
     return SE_OK;
 }
 
