@@ -636,7 +636,7 @@ __global__ void k_bin_place(const int4* __restrict__ slot, const int* __restrict
 // of the loads of 16 warps per SM; parts of 32 or 64 particles leave more
 // CTAs but more windows to clear and add: 244 and 210 us).
 constexpr int SCATTER_SPLIT = 128;
-constexpr int WINDOW_MAX_P = 22;   // (P + 7)^3 doubles fit shared memory
+constexpr int WINDOW_MAX_P = 16;   // two windows of (P + 7)^3 doubles fit an SM
 
 static size_t window_bytes(int P) { return sizeof(double) * (size_t)(P + 7) * (P + 7) * (P + 7); }
 
@@ -1048,11 +1048,27 @@ static int group_by_bin(Stager& s, const int* idx, const SE_FGG_params* p, const
     return SE_OK;
 }
 
-// Grouping takes three launches, 13 us; a particle's stencil cost 12 ns in the
-// gather (30,000 particles, P = 16, force: 370 us in the caller's order and
-// one load at a time, 231 us grouped and eight loads ahead, 165 us with P
-// compiled in), so it pays from a few thousand particles on.
-constexpr int GROUP_MIN_N = 4096;
+// Whether the particles are grouped for a gather.  Grouping takes three
+// launches, 13 us; the gather of 30,000 particles at P = 16 (1.2e8 stencil cells)
+// took 370 us in the caller's order and one load at a time, 231 us grouped and
+// eight loads ahead, 165 us with P compiled in.
+static bool grouped(const SE_FGG_params* p)
+{
+    return (double)p->N * p->P * p->P * p->P >= 1.6e7;
+}
+
+// Whether a scatter goes through shared-memory windows: where they have far
+// fewer cells to clear and add than the particles' stencils (P = 16, all step
+// calls of a pass: 4,200 particles, M = 48, 2.8 times fewer, 337 -> 289 us;
+// 60,000, M = 128, 3.5 times, 2,053 -> 965 us; 6,000, M = 64, P = 12, 1.5 times,
+// no gain), and not where one window fills an SM (10,000, M = 45, P = 20, 5.6
+// times fewer: 814 us, without 614).
+static bool windowed(const SE_FGG_params* p, const StencilBins& B)
+{
+    const double W = p->P + BIN - 1, P = p->P;
+    return grouped(p) && p->P <= WINDOW_MAX_P &&
+           W * W * W * B.count * 2.0 < (double)p->N * P * P * P;
+}
 
 static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params* p,
                          int force_order)
@@ -1070,11 +1086,8 @@ static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params
     const double* zz = (const double*)s.use(w->zz, NP * 8, true, false);
     const int* idx = (const int*)s.use(w->idx, 4 * (size_t)p->N, true, false);
     SE_TRY(s.copy_in());
-    // through shared-memory windows where they have fewer cells to add to H
-    // than the particles' stencils
     const StencilBins B(p);
-    const double W = p->P + BIN - 1;
-    if (p->N >= GROUP_MIN_N && p->P <= WINDOW_MAX_P && W * W * W * B.count < (double)p->N * P3) {
+    if (windowed(p, B)) {
         const int* off;
         const int2* order;
         SE_TRY(group_by_bin(s, idx, p, B, &off, &order));
@@ -1156,7 +1169,7 @@ static int do_int_split(double* phi, const SE_FGG_work* w, const SE_FGG_params* 
     const double h3 = p->h * p->h * p->h;
     const int* off;
     const int2* order = nullptr;
-    if (p->N >= GROUP_MIN_N) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
+    if (grouped(p)) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
     const auto fn = p->P == 16   ? k_int_split<16>
                     : p->P == 12 ? k_int_split<12>
                     : p->P == 8  ? k_int_split<8>
@@ -1208,7 +1221,7 @@ static int do_int_split_force(double* force, const SE_state* st, const SE_FGG_wo
     const double h3 = p->h * p->h * p->h;
     const int* off;
     const int2* order = nullptr;
-    if (p->N >= GROUP_MIN_N) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
+    if (grouped(p)) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
     const auto fn = p->P == 16   ? k_int_split_force<16>
                     : p->P == 12 ? k_int_split_force<12>
                     : p->P == 8  ? k_int_split_force<8>

@@ -1,4 +1,4 @@
-"""The reference step calls on particles grouped by bin (from 4,096 particles
+"""The reference step calls on particles grouped by bin (from 1.6e7 stencil cells
 on): the scatter through shared-memory windows and the gathers in grouped
 order against the oracle, at the edges of their dispatch: stencils with and
 without a compiled-in P, the largest window, one more than it, a bin of more
@@ -26,9 +26,9 @@ def F():
     return fgg
 
 
-@pytest.mark.parametrize("N,M,P,clusters", [(4095, 32, 16, 0), (4096, 32, 16, 0), (5001, 20, 8, 0),
-                                            (4500, 24, 12, 2), (6000, 27, 13, 0), (4200, 16, 21, 0),
-                                            (4100, 18, 22, 1), (4100, 18, 23, 0), (4096, 33, 3, 0)])
+@pytest.mark.parametrize("N,M,P,clusters", [(3906, 32, 16, 0), (3907, 32, 16, 0), (31_251, 20, 8, 0),
+                                            (9300, 24, 12, 2), (7300, 27, 13, 0), (1800, 16, 21, 0),
+                                            (1600, 18, 22, 1), (600_000, 33, 3, 0), (500, 16, 32, 0)])
 @pytest.mark.parametrize("force", [False, True])
 def test_grouped_steps_equal_oracle(F, N, M, P, clusters, force):
     import oracle as O
@@ -65,7 +65,7 @@ def test_grouped_scatter_skips_stencils_outside(F):
     import oracle as O
     import torch
     from se_fast_gridding_b200._lib import SEError
-    N, M, P = 5000, 24, 12
+    N, M, P = 9400, 24, 12
     x, q = O.synthetic_system(N, 1.0, seed=3, charges="uniform")
     m = 0.95 * np.sqrt(O.PI * P)
     _, p = F.fcn_params(M, P, 1.0, 4.0, m, N)
