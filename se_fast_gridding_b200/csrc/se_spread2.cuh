@@ -18,19 +18,34 @@
 // order, keeps the particles whose stencil meets the block and sorts them
 // into three x classes -- the particle's x row in the tile meets both 8-cell
 // halves, the low half only or the high half only -- one list ring each.
-// Whenever a class holds a group (one particle per lane) the warp streams it
+// Whenever a class holds a group the warp streams it
 // through two shared-memory stages that cp.async fills from the factor rows
 // while the warp works on the other: the x tile row (of a one-half class,
-// that half), the warp's 8 y and 8 z entries and the charge.  Each lane adds
-// px[x] * (q py[y] pz[z]) into the 16 x 2 cells of its (y, z) and
-// (y, z + 1), or the 8 x 2 of the class's half: a one-half group costs half
-// the FMAs of a full one, and a particle is a one-half particle in about
-// half of the tiles it meets at P = 16 (more at smaller P).  Every cell
-// belongs to one lane of one CTA: no atomics and a fixed order of summation
-// (the groups' order, which depends only on the block's candidate list).
-// FP32: packed FP32 pair FMAs on the cells, and after every 512 of the
-// warp's particles the FP32 sums are added into the FP64 grid in place (the
-// first time stored), which the lane alone reads and writes.
+// that half), the warp's 8 y and 8 z entries and the charge, consecutive lanes
+// copying consecutive pieces of a row; the next 32 candidates' corners are
+// loaded meanwhile.  (With a particle's pieces copied by one lane, and the
+// corners loaded when they were needed, a group's set-up took as long as its
+// sums: 100,000 particles, M = 128, P = 16, stage 0.130 -> 0.116 ms; 16M
+// clustered, M = 512, P = 12, 11.0 -> 10.1 ms; 256 systems of M = 64 2.37 ->
+// 2.10 ms.)  A one-half group costs half the FMAs of a full one, and a particle
+// is a one-half particle in about half of the tiles it meets at P = 16 (more at
+// smaller P).  Every cell belongs to one lane of one CTA: no atomics and a fixed
+// order of summation (the groups' order, which depends only on the block's
+// candidate list).
+// FP32: each lane adds px[x] * (q py[y] pz[z]) into the 16 x 2 cells of its
+// (y, z) and (y, z + 1), or the 8 x 2 of the class's half, with packed FP32 pair
+// FMAs, and after every 512 of the warp's particles the FP32 sums are added into
+// the FP64 grid in place (the first time stored), which the lane alone reads
+// and writes.
+// FP64: matrix instructions, 4 particles onto 8 x by 8 z cells of one y, with
+// the cells' sums in the accumulators (64 registers).  They run at the rate of
+// scalar FP64 FMAs but need a fraction of the instructions and shared-memory
+// loads: 100,000 particles, M = 128, P = 16 0.240 -> 0.142 ms (the matrix unit's
+// share 0.066 ms, 0.094 with the products that feed it); 1M, M = 256, P = 12 1.10
+// -> 0.63 ms, P = 8 0.59 -> 0.33 ms; 2M clustered 3.49 -> 2.23 ms.  (For FP32 the
+// same products on FP64 units, 0.145 ms, or on BF16 units with 24 bits in three
+// parts, 0.148 ms, lose to packed FMAs: splitting the operands costs more
+// instructions than the FMAs.)
 //
 // Crowded tiles are split.  Each warp's candidate list is cut into parts of
 // at most S2_CAP candidates; k_tile_parts counts the candidates of each
@@ -53,22 +68,13 @@
 #endif
 constexpr int S2_CAP = SE_S2_CAP;   // candidates per part of a warp's list
 constexpr int S2_WARPS = 4;   // warp blocks per tile
-// warps per CTA: a tile's four warp blocks run as S2_WARPS / S2_CTA_WARPS
-// CTAs (the warps are independent), so that the SMs share out the blocks
-// more evenly (two CTAs of 2 warps per tile against one of 4: C2 spread
-// 0.135 -> 0.128 ms, C3 2.33 -> 2.26 ms, C5 12.7 -> 11.6 ms)
-#ifndef SE_S2_CTA_WARPS
-#define SE_S2_CTA_WARPS 2
-#endif
-constexpr int S2_CTA_WARPS = SE_S2_CTA_WARPS;
-static_assert(S2_WARPS % S2_CTA_WARPS == 0, "a tile's warp blocks split evenly into CTAs");
-// grids of at least S2_ONE_WARP_TILES tiles (the 5-CTA build) run one warp
-// per CTA instead (the M = 512 clustered spread 11.48 -> 11.13 ms; smaller
-// grids measured better with two)
-#ifndef SE_S2_ONE_WARP_TILES
-#define SE_S2_ONE_WARP_TILES 32768
-#endif
-constexpr int S2_ONE_WARP_TILES = SE_S2_ONE_WARP_TILES;
+// warps per CTA: a tile's four warp blocks run as S2_WARPS / CW CTAs (the warps
+// are independent), so that the SMs share out the blocks more evenly: one warp
+// in FP32 (against two: 1M uniform, M = 256, P = 12 0.548 -> 0.529 ms, 256
+// systems of M = 64 2.10 -> 2.05 ms, 16M clustered no difference), two in FP64
+// (2M clustered 2.28 -> 2.23 ms)
+template <typename Acc>
+constexpr int s2_cta_warps() { return sizeof(Acc) == 4 ? 1 : 2; }
 constexpr int S2_LIST = 64;    // per-class list ring: >= group - 1 + 32
 constexpr int S2_SEGS = 64;    // bin segments reaching a warp's block: <= 5 x 4 x 2 for P <= 16
 constexpr int S2_FOLD = 512;   // FP32 partial sums cover this many of a warp's particles
@@ -79,7 +85,7 @@ constexpr int S2_UNROLL = SE_S2_UNROLL;   // particles per unrolled pass of a gr
 // FP32 CTAs per SM the kernel is compiled for: 5 (96 registers) where the
 // tiles outnumber 4 CTAs per SM, 4 (128 registers) where all of them are
 // resident at once either way; FP64: 3
-constexpr int S2_BLOCKS_MANY = 5, S2_BLOCKS_FEW = 4, S2_BLOCKS_FP64 = 3;
+constexpr int S2_BLOCKS_MANY = 5, S2_BLOCKS_FEW = 4, S2_BLOCKS_FP64 = 4;
 
 // particles a warp stages at once: one per lane (FP32), half a warp (FP64)
 template <typename Acc>
@@ -93,10 +99,25 @@ struct Spread2Stage {
     double q[s2_group<Acc>()];
 };
 
+// Where entry x of staged particle k's x row and entry z of its y and z rows
+// lie in the row: in FP64 moved (whole 32-byte groups) so that a warp's operand
+// loads, 8 entries of 4 consecutive particles, fall in distinct banks.
+template <typename Acc>
+__device__ __forceinline__ int s2_px(int k, int x)
+{
+    return sizeof(Acc) == 4 ? x : x ^ ((k & 3) << 2);
+}
+
+template <typename Acc>
+__device__ __forceinline__ int s2_pz(int k, int z)
+{
+    return sizeof(Acc) == 4 ? z : z ^ (((k >> 1) & 1) << 2);
+}
+
 template <typename Acc, int CW>
 struct Spread2Smem {
     Spread2Stage<Acc> stage[CW][2];
-    int2 list[CW][S2_CLASSES][S2_LIST];   // (particle, packed grid index)
+    unsigned list[CW][S2_CLASSES][S2_LIST];   // 8 particle + 4 hx + 2 hy + hz (the halves of its rows)
     int seg_beg[CW][S2_SEGS];
     int seg_pre[CW][S2_SEGS];
 };
@@ -111,6 +132,21 @@ __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
+
+// 16 bytes, or 16 zero bytes where !on (gsrc is then not read)
+__device__ __forceinline__ void cp_async16_or_zero(void* sdst, const void* gsrc, bool on)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(on ? 16 : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cp_async8_or_zero(void* sdst, const void* gsrc, bool on)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gsrc), "r"(on ? 8 : 0)
+                 : "memory");
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -185,56 +221,64 @@ struct Spread2Accum<float> {
     }
 };
 
+// FP64: the cells of the warp's block as the matrix instructions spread them
+// over a warp: with g = lane / 4 and t = lane % 4, x in {g, g + 8}, every y, z in
+// {2 t, 2 t + 1}.  One instruction adds 4 particles to 8 x by 8 z cells of one y:
+// D[x][z] += px[x] (py[y] (q pz[z])).
 template <>
 struct Spread2Accum<double> {
-    double a[16], b[16];
+    double v[8][4];   // [y][x = g: z, z + 1; x = g + 8: z, z + 1]
     __device__ __forceinline__ void zero()
     {
 #pragma unroll
-        for (int x = 0; x < 16; x++) a[x] = b[x] = 0.0;
-    }
-    __device__ __forceinline__ void add(const double* px, double c0, double c1)
-    {
-        const double2* p2 = reinterpret_cast<const double2*>(px);
+        for (int y = 0; y < 8; y++)
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const double2 w = p2[m];
-            a[2 * m] = fma(w.x, c0, a[2 * m]);
-            a[2 * m + 1] = fma(w.y, c0, a[2 * m + 1]);
-            b[2 * m] = fma(w.x, c1, b[2 * m]);
-            b[2 * m + 1] = fma(w.y, c1, b[2 * m + 1]);
+            for (int k = 0; k < 4; k++) v[y][k] = 0.0;
+    }
+    // staged particles i .. i + 3, particle i + t the contraction's element t;
+    // HALVES bit 0: x in [0, 8), bit 1: x in [8, 16)
+    template <int HALVES>
+    __device__ __forceinline__ void add(const Spread2Stage<double>& st, int i, int g, int t)
+    {
+        const int k = i + t;
+        const double a0 = (HALVES & 1) ? st.px[k][s2_px<double>(t, g)] : 0.0;
+        const double a1 = (HALVES & 2) ? st.px[k][s2_px<double>(t, g + 8)] : 0.0;
+        const double pz = st.q[k] * st.pz[k][s2_pz<double>(t, g)];
+#pragma unroll
+        for (int y = 0; y < 8; y += 2) {
+            const double2 py = *reinterpret_cast<const double2*>(&st.py[k][s2_pz<double>(t, y)]);
+            const double b0 = py.x * pz, b1 = py.y * pz;
+            if (HALVES & 1) mma_f64(v[y][0], v[y][1], a0, b0);
+            if (HALVES & 2) mma_f64(v[y][2], v[y][3], a1, b0);
+            if (HALVES & 1) mma_f64(v[y + 1][0], v[y + 1][1], a0, b1);
+            if (HALVES & 2) mma_f64(v[y + 1][2], v[y + 1][3], a1, b1);
         }
     }
-    template <int H>
-    __device__ __forceinline__ void add_half(const double* px, double c0, double c1)
+    // the first n particles of the stage (zero rows up to a multiple of 4)
+    template <int HALVES>
+    __device__ __forceinline__ void add_group(const Spread2Stage<double>& st, int n, int g, int t)
     {
-        const double2* p2 = reinterpret_cast<const double2*>(px);
+        constexpr int G = s2_group<double>();
+        if (n == G) {
 #pragma unroll
-        for (int m = 4 * H; m < 4 * H + 4; m++) {
-            const double2 w = p2[m];
-            a[2 * m] = fma(w.x, c0, a[2 * m]);
-            a[2 * m + 1] = fma(w.y, c0, a[2 * m + 1]);
-            b[2 * m] = fma(w.x, c1, b[2 * m]);
-            b[2 * m + 1] = fma(w.y, c1, b[2 * m + 1]);
+            for (int i = 0; i < G; i += 4) add<HALVES>(st, i, g, t);
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < n; i += 4) add<HALVES>(st, i, g, t);
         }
     }
-    __device__ __forceinline__ void store(double* cell0, long long plane) const
+    // cell (x, y, z) at cell0 + x plane + y row + z, cell0 that of the lane's
+    // first x and z
+    __device__ __forceinline__ void store(double* cell0, long long plane, int row) const
     {
 #pragma unroll
-        for (int x = 0; x < 16; x++)
-            *reinterpret_cast<double2*>(cell0 + x * plane) = make_double2(a[x], b[x]);
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int y = 0; y < 8; y++)
+                *reinterpret_cast<double2*>(cell0 + 8 * h * plane + y * row) =
+                    make_double2(v[y][2 * h], v[y][2 * h + 1]);
     }
 };
-
-// Half h in {0, 1} of the home tile t0 = g / 16 that is tile ti, or -1 when
-// the stencil [g, g + P) misses tile ti (nt tiles per axis, periodic).
-__device__ __forceinline__ int tile_half(int g, int ti, int nt, int P)
-{
-    int h = ti - (g >> 4);
-    if (h < 0) h += nt;
-    if (h == 0) return 0;
-    return (h == 1 && (g & 15) + P > 16) ? 1 : -1;
-}
 
 // The bins whose particles may reach block (wy, wz) of a tile at corner
 // (x0, y0, z0) -- x: the tile's 16 cells, y and z: the block's 8 -- as
@@ -372,7 +416,7 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
 }
 
 // CW warps per CTA (S2_WARPS / CW CTAs per part of a tile)
-template <typename Acc, int BLOCKS, int CW = S2_CTA_WARPS>
+template <typename Acc, int BLOCKS, int CW = s2_cta_warps<Acc>()>
 __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     const SysDev* __restrict__ sys, const int* __restrict__ tile_sys,
     const double4* __restrict__ srec, const int* __restrict__ sg,
@@ -416,7 +460,6 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     const int warp = sub * CW + lw;   // the warp block of the tile
     const int wy = warp >> 1, wz = warp & 1;
     const int ly = lane >> 2, lz = (lane & 3) * 2;
-    const unsigned ybits = 0xFFu << (8 * wy), zbits = 0xFFu << (8 * wz);
 
     // ---- the bin segments reaching this warp's block (at most 5 x 4 x 2) and
     // their prefix: the warp's own candidate list, in segment order
@@ -447,16 +490,16 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     }
     __syncwarp();   // the warps are independent from here on
 
-    const unsigned pmask = (1u << P) - 1u;   // P <= 16
     const unsigned lanes_before = (1u << lane) - 1u;
     double* gs = grid + S.grid_off;
     const long long gplane = (long long)M * M;
-    // part 0 sums into the grid, the others into their slab slot
-    // (cells [x][y][z] of the tile, 16^3)
+    // part 0 sums into the grid, the others into their slab slot (cells
+    // [x][y][z] of the tile, 16^3); cell0: the lane's first cell
     const long long plane = ipart == 0 ? gplane : 256;
-    double* cell0 =
-        ipart == 0 ? gs + (long long)x0 * gplane + (long long)(y0 + 8 * wy + ly) * M + z0 + 8 * wz + lz
-                  : slab + (long long)(slot0 + ipart - 1) * 4096 + (8 * wy + ly) * 16 + 8 * wz + lz;
+    const int row = ipart == 0 ? M : 16;
+    double* cell0 = (ipart == 0 ? gs + (long long)x0 * gplane + (long long)y0 * M + z0
+                                : slab + (long long)(slot0 + ipart - 1) * 4096) +
+                    (long long)(8 * wy) * row + 8 * wz + lz + (FOLD ? (long long)ly * row : ly * plane);
     // this part's candidates: [cbeg, cend) of the warp's list
     const int cbeg = ipart * S2_CAP, cend = min(total, cbeg + S2_CAP);
 
@@ -470,26 +513,40 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     int cpos = cbeg, buf = 0, pending = 0, pcls = 0, since_fold = 0;
     int seg = 0;   // the segment holding candidate cpos
     while (seg + 1 < nseg && seg_pre[seg + 1] <= cpos) seg++;
+    // the lane's candidate of the 32 at cpos, loaded one round ahead
+    int part = 0, pk = 0;
+    auto fetch = [&] {
+        const int pos = cpos + lane;
+        int sl = seg;   // this lane's segment, found forward
+        if (pos < cend) {
+            while (sl + 1 < nseg && seg_pre[sl + 1] <= pos) sl++;
+            part = seg_beg[sl] + (pos - seg_pre[sl]);
+            pk = sg[part];
+        }
+        seg = __reduce_max_sync(0xffffffffu, sl);
+    };
+    fetch();
     bool written = false;
     for (;;) {
         // ---- list until some class holds a group (or every remaining
         // candidate is listed), each class in candidate order
         while (!(cnt & FULL) && cpos < cend) {
-            const int pos = cpos + lane;
-            int part = -1, pk = 0, cls = -1, sl = seg;   // this lane's segment, found forward
-            if (pos < cend) {
-                while (sl + 1 < nseg && seg_pre[sl + 1] <= pos) sl++;
-                part = seg_beg[sl] + (pos - seg_pre[sl]);
-                pk = sg[part];
-                // the stencil's cells in this tile, as 16-bit masks per axis
-                const int gx = g_of(pk, 0), gy = g_of(pk, 1), gz = g_of(pk, 2);
-                const int hx = tile_half(gx, tix, nt, P);
-                const int hy = tile_half(gy, tiy, nt, P), hz = tile_half(gz, tiz, nt, P);
-                const unsigned xm = ((pmask << (gx & 15)) >> (16 * max(hx, 0))) & 0xFFFFu;
-                const bool meets = hx >= 0 && hy >= 0 && hz >= 0 &&
-                                   ((((pmask << (gy & 15)) >> (16 * hy)) & 0xFFFFu) & ybits) &&
-                                   ((((pmask << (gz & 15)) >> (16 * hz)) & 0xFFFFu) & zbits);
-                if (meets) cls = (xm & 0xFFu) ? ((xm & 0xFF00u) ? 0 : 1) : 2;
+            int cls = -1;
+            unsigned entry = 0;
+            if (cpos + lane < cend) {
+                // per axis: which tile after the home tile this one is, and
+                // the stencil's entry at the tile's (block's) first cell
+                int hx = tix - (g_of(pk, 0) >> 4), hy = tiy - (g_of(pk, 1) >> 4), hz = tiz - (g_of(pk, 2) >> 4);
+                hx += hx < 0 ? nt : 0;
+                hy += hy < 0 ? nt : 0;
+                hz += hz < 0 ? nt : 0;
+                const int ex = 16 * hx - (g_of(pk, 0) & 15);
+                const int ey = 16 * hy - (g_of(pk, 1) & 15) + 8 * wy, ez = 16 * hz - (g_of(pk, 2) & 15) + 8 * wz;
+                // 8 cells from entry e on meet the stencil's entries [0, P)
+                auto meets = [&](int e) { return (unsigned)(e + 7) < (unsigned)(P + 7); };
+                const bool lo = meets(ex), hi = meets(ex + 8);
+                if (meets(ey) && meets(ez)) cls = lo ? (hi ? 0 : 1) : (hi ? 2 : -1);
+                entry = ((unsigned)part << 3) | (hx << 2) | (hy << 1) | hz;
             }
             const unsigned k0 = __ballot_sync(0xffffffffu, cls == 0);
             const unsigned k1 = __ballot_sync(0xffffffffu, cls == 1);
@@ -498,11 +555,11 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
                 const unsigned kc = cls == 0 ? k0 : (cls == 1 ? k1 : k2);
                 const int sh = 8 * cls;
                 sm.list[lw][cls][((ring >> sh) + (cnt >> sh) + __popc(kc & lanes_before)) &
-                                   (S2_LIST - 1)] = make_int2(part, pk);
+                                   (S2_LIST - 1)] = entry;
             }
             cnt += __popc(k0) | (__popc(k1) << 8) | (__popc(k2) << 16);
             cpos += 32;
-            seg = __reduce_max_sync(0xffffffffu, sl);
+            fetch();
         }
         __syncwarp();   // list entries visible to the warp
         // ---- the class to stage: a full group if some class has one (the
@@ -512,39 +569,36 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
         const int sh = 8 * cls;
         const int avail = (cnt >> sh) & 0xFF;
         const int head = (ring >> sh) & (S2_LIST - 1);
-        const int2* list = sm.list[lw][cls];
-        // ---- stage the next group of the class: lane l < n copies its
-        // particle head + l (of a one-half class, that half of the x row)
+        const unsigned* list = sm.list[lw][cls];
+        // ---- stage the next group of the class: the x tile rows (of a
+        // one-half class, that half), the block's 8 y and 8 z entries and the
+        // charges, zeros past the group's n particles; consecutive lanes copy
+        // consecutive 16-byte pieces of a row
         const int n = min(G, avail);
         if (n > 0) {
             Spread2Stage<Acc>& st = sm.stage[lw][buf];
-            if (lane < n) {
-                const int2 e = list[(head + lane) & (S2_LIST - 1)];
-                const int hx = tile_half(g_of(e.y, 0), tix, nt, P);
-                const int hy = tile_half(g_of(e.y, 1), tiy, nt, P);
-                const int hz = tile_half(g_of(e.y, 2), tiz, nt, P);
-                const Acc* r = rows + (long long)e.x * 96;
-                if (cls == 0) {
+            constexpr int C8 = 8 / V, C16 = 16 / V;   // pieces per 8 and 16 entries
+            if (cls == 0) {
 #pragma unroll
-                    for (int k = 0; k < 16; k += V) cp_async16(&st.px[lane][k], r + 16 * hx + k);
-                } else {
+                for (int i0 = 0; i0 < G; i0 += 32 / C16) {
+                    const int i = i0 + lane / C16, k = V * (lane % C16);
+                    const unsigned e = i < n ? list[(head + i) & (S2_LIST - 1)] : 0u;
+                    cp_async16_or_zero(&st.px[i][s2_px<Acc>(i, k)],
+                                       rows + (long long)(e >> 3) * 96 + 4 * (e & 4) + k, i < n);
+                }
+            }
+#pragma unroll
+            for (int i0 = 0; i0 < G; i0 += 32 / C8) {
+                const int i = i0 + lane / C8, k = V * (lane % C8);
+                const unsigned e = i < n ? list[(head + i) & (S2_LIST - 1)] : 0u;
+                const Acc* r = rows + (long long)(e >> 3) * 96 + k;
+                if (cls != 0) {
                     const int o = 8 * (cls - 1);
-#pragma unroll
-                    for (int k = 0; k < 8; k += V) cp_async16(&st.px[lane][o + k], r + 16 * hx + o + k);
+                    cp_async16_or_zero(&st.px[i][s2_px<Acc>(i, o + k)], r + 4 * (e & 4) + o, i < n);
                 }
-#pragma unroll
-                for (int k = 0; k < 8; k += V) {
-                    cp_async16(&st.py[lane][k], r + 32 + 16 * hy + 8 * wy + k);
-                    cp_async16(&st.pz[lane][k], r + 64 + 16 * hz + 8 * wz + k);
-                }
-                cp_async8(&st.q[lane], &srec[e.x].w);
-            } else if (lane < G) {   // a short group: zero rows up to G (FP64: 16),
-                                     // so every group sums G rows
-#pragma unroll
-                for (int k = 0; k < 16; k++) st.px[lane][k] = Acc(0);
-#pragma unroll
-                for (int k = 0; k < 8; k++) st.py[lane][k] = st.pz[lane][k] = Acc(0);
-                st.q[lane] = 0.0;
+                cp_async16_or_zero(&st.py[i][s2_pz<Acc>(i, k)], r + 32 + 8 * (e & 2) + 8 * wy, i < n);
+                cp_async16_or_zero(&st.pz[i][s2_pz<Acc>(i, k)], r + 64 + 16 * (e & 1) + 8 * wz, i < n);
+                if (k == 0) cp_async8_or_zero(&st.q[i], &srec[e >> 3].w, i < n);
             }
             cp_async_commit();
             cnt -= (unsigned)n << sh;
@@ -557,34 +611,41 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
             else cp_async_wait<0>();
             __syncwarp();
             Spread2Stage<Acc>& st = sm.stage[lw][buf ^ 1];
-            // lane i scales its particle's 8 y entries by the charge, once
-            if (lane < pending) {
-                const Acc qv = (Acc)st.q[lane];
+            if constexpr (FOLD) {
+                // lane i scales its particle's 8 y entries by the charge, once
+                if (lane < pending) {
+                    const Acc qv = (Acc)st.q[lane];
 #pragma unroll
-                for (int k = 0; k < 8; k++) st.py[lane][k] = st.py[lane][k] * qv;
-            }
-            __syncwarp();
-            // every group holds G rows (a short one padded with zeros, which
-            // add exact zeros): one unrolled pass per class with constant
-            // offsets; a one-half class touches the lane's 8 x 2 cells of its half
-            if (pcls == 0) {
-#pragma unroll S2_UNROLL
-                for (int i = 0; i < G; i++) {
-                    const Acc y = st.py[i][ly];
-                    acc.add(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
+                    for (int k = 0; k < 8; k++) st.py[lane][k] = st.py[lane][k] * qv;
                 }
-            } else if (pcls == 1) {
+                __syncwarp();
+                // every group holds G rows (a short one padded with zeros, which
+                // add exact zeros): one unrolled pass per class with constant
+                // offsets; a one-half class touches the lane's 8 x 2 cells of its half
+                if (pcls == 0) {
 #pragma unroll S2_UNROLL
-                for (int i = 0; i < G; i++) {
-                    const Acc y = st.py[i][ly];
-                    acc.template add_half<0>(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
+                    for (int i = 0; i < G; i++) {
+                        const Acc y = st.py[i][ly];
+                        acc.add(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
+                    }
+                } else if (pcls == 1) {
+#pragma unroll S2_UNROLL
+                    for (int i = 0; i < G; i++) {
+                        const Acc y = st.py[i][ly];
+                        acc.template add_half<0>(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
+                    }
+                } else {
+#pragma unroll S2_UNROLL
+                    for (int i = 0; i < G; i++) {
+                        const Acc y = st.py[i][ly];
+                        acc.template add_half<1>(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
+                    }
                 }
             } else {
-#pragma unroll S2_UNROLL
-                for (int i = 0; i < G; i++) {
-                    const Acc y = st.py[i][ly];
-                    acc.template add_half<1>(st.px[i], y * st.pz[i][lz], y * st.pz[i][lz + 1]);
-                }
+                const int t4 = lane & 3;
+                if (pcls == 0) acc.template add_group<3>(st, pending, ly, t4);
+                else if (pcls == 1) acc.template add_group<1>(st, pending, ly, t4);
+                else acc.template add_group<2>(st, pending, ly, t4);
             }
             if constexpr (FOLD) {
                 since_fold += pending;
@@ -606,7 +667,7 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     if constexpr (FOLD) {
         if (since_fold > 0 || !written) acc.fold(cell0, plane, !written);
     } else {
-        acc.store(cell0, plane);
+        acc.store(cell0, plane, row);
     }
 
     // ---- a split tile: the part that finishes last adds the slabs into the
