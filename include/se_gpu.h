@@ -94,7 +94,8 @@ int se_plan_create(se_plan* plan, const se_config* cfg);
 int se_plan_destroy(se_plan plan);
 
 /* Kernel paths (se_plan_create_ex): which spread and interpolation kernels a
- * plan runs.  SE_PATH_TILE_SPREAD and SE_PATH_PAIR_INTERP need M a multiple
+ * plan runs.  SE_PATH_TILE_SPREAD and SE_PATH_PAIR_INTERP (the kernels that read
+ * tile-aligned factor rows) need M a multiple
  * of 16, M >= 32 and P <= 16; SE_PATH_RUNTIME_P turns off the interpolation
  * kernels specialised for P = 8, 12, 16 (21).  SE_PATH_DEFAULT is what
  * se_plan_create does (the tile spread where it applies, the pair
@@ -105,7 +106,7 @@ int se_plan_destroy(se_plan plan);
  * the environment variable SE_GPU_TUNE_FILE set, in that file.  Every path
  * meets the same accuracy; different paths sum in different orders, so their
  * results differ in the last bits.  se_plan_device_bytes reports the default
- * path; a path mixing tile and general kernels holds 3P more factors per
+ * path; a path mixing kernels on tile-aligned and other rows holds 3P more factors per
  * particle. */
 #define SE_PATH_DEFAULT (-1)
 #define SE_PATH_TUNE (-2)

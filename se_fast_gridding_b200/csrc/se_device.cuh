@@ -42,12 +42,20 @@ __host__ __device__ inline bool spread2_eligible(int M, int P)
 }
 
 // A system's kernel path (SysDev::path): which spread and interpolation run.
-constexpr int PATH_TILE_SPREAD = 1;    // k_spread2 (else k_spread)
+constexpr int PATH_TILE_SPREAD = 1;    // k_spread2 on tile-aligned rows
 constexpr int PATH_PAIR_INTERP = 2;    // k_interp2 or k_interp3 on tile-aligned rows
 constexpr int PATH_RUNTIME_P = 4;      // interpolation without the P-unrolled variants
 constexpr int PATH_RADIX_SORT = 8;     // the batch sorts with the radix passes (se_sort.cu)
 constexpr int PATH_FFT3 = 16;          // the batch's FP64 FFTs through se_fft.cuh (not cuFFT)
 constexpr int PATH_BIN_WINDOWS = 32;   // k_interp2 stages one window per bin (not per z pair)
+
+// Whether a system off the whole tiles spreads by k_spread2 on its P-wide
+// factor rows: where no cell lies in a stencil twice as seen from one 16^3 tile
+// (M >= P + 15); k_spread serves the smaller grids.
+__host__ __device__ inline bool spread2_general(int path, int M, int P)
+{
+    return !(path & PATH_TILE_SPREAD) && M >= P + 15;
+}
 
 // Whether k_interp3 serves a system (else k_interp2 on the path with
 // PATH_PAIR_INTERP, k_interp without).  Measured on B200, interpolation stage:

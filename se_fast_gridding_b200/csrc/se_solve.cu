@@ -13,8 +13,8 @@
 //   k_factors   each particle's separable Gaussian factors, FGG recurrence
 //               (tile-aligned rows for the tile kernels)
 //   spread      k_tile_parts + k_spread2, one CTA per part of a 16^3 tile,
-//               the fold fused (se_spread2.cuh), for grids of whole tiles and
-//               P <= 16; k_spread (se_spread.cuh) for the others
+//               the fold fused (se_spread2.cuh); k_spread (se_spread.cuh) on
+//               the smallest grids (M < P + 15)
 //   cuFFT D2Z, k_scale (Z of scaling(), SE_general.c:145-175, applied to the
 //               half spectrum as product_rc does, SE_general.c:336-362), Z2D
 //   interp      one launch per stencil and mode of the batch, the unfold fused:
@@ -34,6 +34,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "se_internal.h"
@@ -419,7 +420,9 @@ struct se_batch_s {
     // resident at once with 4 per SM (more registers, the same sums), else
     // S2_BLOCKS_MANY
     bool spread2_few = false;
-    bool any_spread1 = false, any_spread2 = false;   // some system on k_spread / k_spread2
+    bool split = false;      // some k_spread2 system may have a tile of several parts
+    // some system on k_spread, on k_spread2 with tile-aligned or P-wide rows
+    bool any_spread1 = false, any_tile_spread = false, any_general_spread = false;
     bool any_interp1 = false, any_interp2 = false;   // on k_interp / with PATH_PAIR_INTERP
     bool runtime_p = false;                          // some system asks for runtime P
     float* grid32 = nullptr;  // FP32 copy of the grids, staged by k_interp2<float>
@@ -557,12 +560,15 @@ static int path_of(const se_system* sys, const int* paths, int i)
     return paths ? paths[i] : default_path(sys[i].M, sys[i].P);
 }
 
-// Slab slots k_spread2 may need for the particles of its systems: a bin is a
-// candidate of at most 2 tiles per axis, so the candidates of all tiles sum
-// to at most 8 N and the parts after each tile's first to 8 N / S2_CAP.
-static int split_slots(long long ntile2)
+// Slab slots k_spread2 may need for a system, the parts after each tile's first:
+// at most the candidates of all its tiles over a part's, the candidates at most N
+// times the tiles that a bin's stencils (FB + P - 1 cells) reach -- 2 per axis on
+// whole tiles, else with a cut tile of one cell among them.
+static long long split_slots(const se_system& s, int path)
 {
-    return (int)(8 * ntile2 / S2_CAP) + 1;
+    if (s.N <= S2_CAP || (!(path & PATH_TILE_SPREAD) && !spread2_general(path, s.M, s.P))) return 0;
+    const long long t = path & PATH_TILE_SPREAD ? 2 : (FB + s.P - 4) / TX + 3;
+    return t * t * t * s.N / split_cap(path, s.N);
 }
 
 static size_t batch_bytes(const se_system* sys, int nsys, int precision, int* nbins_out,
@@ -595,11 +601,9 @@ static size_t batch_bytes(const se_system* sys, int nsys, int precision, int* nb
     }
     if (plain) b += (size_t)ntot * 3 * maxP * (precision == SE_FP32 ? 4 : 8);
     if (rows) b += (size_t)ntot * 3 * 32 * (precision == SE_FP32 ? 4 : 8);
-    long long ntile2 = 0;
-    for (int i = 0; i < nsys; i++)
-        if (path_of(sys, paths, i) & PATH_TILE_SPREAD) ntile2 += sys[i].N;
-    if (ntile2 > 0 || rows)
-        b += (size_t)split_slots(ntile2) * 4096 * 8 + (size_t)(2 * ntiles + 2) * 4;
+    long long slots = 1;
+    for (int i = 0; i < nsys; i++) slots += split_slots(sys[i], path_of(sys, paths, i));
+    if (slots > 1) b += (size_t)slots * 4096 * 8 + (size_t)(2 * ntiles + 2) * 4;
     if ((pair && precision == SE_FP32) || fft32) b += (size_t)grid * 4;   // FP32 grids
     b += std::max(sort_scratch_bytes((int)ntot, (int)std::max<long long>(nbins, 1)),
                   bsort_scratch_bytes((int)std::max<long long>(nbins, 1)));
@@ -983,7 +987,10 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
     int window_P = 0;   // the largest stencil of the k_interp systems
     for (int i = 0; i < nsys; i++) {
         const int path = b->host_sys[i].path;
-        (path & PATH_TILE_SPREAD ? b->any_spread2 : b->any_spread1) = true;
+        if (path & PATH_TILE_SPREAD) b->any_tile_spread = true;
+        else if (spread2_general(path, systems[i].M, systems[i].P)) b->any_general_spread = true;
+        else b->any_spread1 = true;
+        if (systems[i].N > S2_CAP) b->split = true;
         if (path & PATH_PAIR_INTERP) b->any_interp2 = true;
         else if (const SysDev& S = b->host_sys[i]; !interp3_better(path, precision, S.M, S.P, S.mode)) {
             b->interp_P = !b->any_interp1 || b->interp_P == S.P ? S.P : 0;
@@ -997,21 +1004,21 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
     }
     if (need_fac) SE_ALLOC(b->fac, nt * 3 * b->PS * (precision == SE_FP32 ? 4 : 8));
     if (need_rows) SE_ALLOC(b->rows, nt * 3 * 32 * (precision == SE_FP32 ? 4 : 8));
-    if (b->any_spread2) {
-        long long ntile2 = 0;
-        for (int i = 0; i < nsys; i++)
-            if (b->host_sys[i].path & PATH_TILE_SPREAD) ntile2 += systems[i].N;
-        b->slab_slots = split_slots(ntile2);
-        SE_ALLOC(b->tile_parts, sizeof(int) * (b->ntiles + 1));
-        SE_ALLOC(b->part_tile, sizeof(int) * (size_t)(b->ntiles + b->slab_slots));
+    if (b->any_tile_spread || b->any_general_spread) {
+        long long slots = 1;
+        for (int i = 0; i < nsys; i++) slots += split_slots(systems[i], b->host_sys[i].path);
+        b->slab_slots = (int)slots;
         SE_ALLOC(b->tile_sys, sizeof(int) * std::max(b->ntiles, 1));
-        {   // every entry a valid tile from the start (k_tile_parts rewrites them per solve)
+        if (b->split) {
+            SE_ALLOC(b->tile_parts, sizeof(int) * (b->ntiles + 1));
+            SE_ALLOC(b->part_tile, sizeof(int) * (size_t)(b->ntiles + b->slab_slots));
+            // every entry a valid tile from the start (k_tile_parts rewrites them per solve)
             const cudaError_t z = cudaMemset(b->part_tile, 0, sizeof(int) * (size_t)(b->ntiles + b->slab_slots));
             if (z != cudaSuccess) return fail(cuda_fail(z, "cudaMemset", __FILE__, __LINE__));
+            SE_ALLOC(b->tile_done, sizeof(int) * std::max(b->ntiles, 1));
+            SE_ALLOC(b->tp_counter, sizeof(unsigned));
+            SE_ALLOC(b->slab, sizeof(double) * 4096 * (size_t)b->slab_slots);
         }
-        SE_ALLOC(b->tile_done, sizeof(int) * std::max(b->ntiles, 1));
-        SE_ALLOC(b->tp_counter, sizeof(unsigned));
-        SE_ALLOC(b->slab, sizeof(double) * 4096 * (size_t)b->slab_slots);
     }
     if ((b->any_interp2 && precision == SE_FP32) || fft32)
         SE_ALLOC(b->grid32, sizeof(float) * (b->grid_elems + 16));
@@ -1100,6 +1107,12 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
         if (a == cudaSuccess)
             a = cudaFuncSetAttribute((const void*)k_spread2<double, S2_BLOCKS_FP64>,
                                      cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+        if (a == cudaSuccess)
+            a = cudaFuncSetAttribute((const void*)k_spread2<float, S2_BLOCKS_FP64, true>,
+                                     cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+        if (a == cudaSuccess)
+            a = cudaFuncSetAttribute((const void*)k_spread2<double, S2_BLOCKS_FP64, true>,
+                                     cudaFuncAttributePreferredSharedMemoryCarveout, carve);
         if (a != cudaSuccess) return fail(cuda_fail(a, "cudaFuncSetAttribute", __FILE__, __LINE__));
     }
     if (b->any_interp1) {
@@ -1168,34 +1181,45 @@ static int run_prepare_sort(se_batch b, const double* x, const double* q, cudaSt
     return run_factors(b, st);
 }
 
+template <typename T, int BLOCKS, bool GEN>
+static int launch_spread2(se_batch b, const void* rows, double* grid, cudaStream_t st)
+{
+    constexpr int CW = s2_cta_warps<T, GEN>();
+    k_spread2<T, BLOCKS, GEN>
+        <<<(b->ntiles + (b->split ? b->slab_slots : 0)) * (S2_WARPS / CW), CW * 32, 0, st>>>(
+            b->sys, b->tile_sys, b->srec, b->sg, static_cast<const T*>(rows), b->PS, b->boff, grid,
+            b->split ? b->tile_parts : nullptr, b->part_tile, b->ntiles, b->tile_done, b->slab, b->slab_slots,
+            b->err);
+    SE_CUDA(cudaGetLastError());
+    LAUNCHED(b);
+    return SE_OK;
+}
+
 static int run_spread(se_batch b, double* grid, cudaStream_t st)
 {
-    // every tile is written by exactly one of the two kernels (by system)
-    if (b->any_spread2) {
+    // every tile is written by exactly one of the kernels (by system)
+    const bool fp32 = b->precision == SE_FP32;
+    if ((b->any_tile_spread || b->any_general_spread) && b->split) {
         // the parts of each tile and each part's tile, then one CTA per part
-        // (at most the bound; the CTAs past the number of parts return at once)
+        // (at most the bound; the CTAs past the number of parts return at once).
+        // A tile has no more candidates than its system has particles: with at
+        // most S2_CAP each there is nothing to split and no need of the count
+        // (0.009 ms of a spread: 3,900 particles, M = 100, P = 8 0.025 -> 0.016 ms)
         const int bound = b->ntiles + b->slab_slots;
         k_tile_parts<<<ceil_div(b->ntiles, TP_TILES), TP_WARPS * 32, 0, st>>>(
             b->sys, b->d_tile_prefix, b->nsys, b->ntiles, b->boff, b->tile_parts, b->tp_counter,
             bound, b->err, b->part_tile);
         SE_CUDA(cudaGetLastError());
         LAUNCHED(b);
-        if (b->precision == SE_FP32)
-            (b->spread2_few ? k_spread2<float, S2_BLOCKS_FEW> : k_spread2<float, S2_BLOCKS_MANY>)
-                <<<bound * (S2_WARPS / s2_cta_warps<float>()), s2_cta_warps<float>() * 32, 0, st>>>(
-                    b->sys, b->tile_sys, b->srec, b->sg,
-                    static_cast<const float*>(b->rows), b->boff, grid, b->tile_parts,
-                    b->part_tile, b->ntiles,
-                    b->tile_done, b->slab, b->slab_slots, b->err);
-        else
-            k_spread2<double, S2_BLOCKS_FP64>
-                <<<bound * (S2_WARPS / s2_cta_warps<double>()), s2_cta_warps<double>() * 32, 0, st>>>(
-                    b->sys, b->tile_sys, b->srec, b->sg,
-                    static_cast<const double*>(b->rows), b->boff, grid, b->tile_parts,
-                    b->part_tile, b->ntiles,
-                    b->tile_done, b->slab, b->slab_slots, b->err);
-        SE_CUDA(cudaGetLastError());
-        LAUNCHED(b);
+    }
+    if (b->any_tile_spread) {
+        if (!fp32) SE_TRY((launch_spread2<double, S2_BLOCKS_FP64, false>(b, b->rows, grid, st)));
+        else if (b->spread2_few) SE_TRY((launch_spread2<float, S2_BLOCKS_FEW, false>(b, b->rows, grid, st)));
+        else SE_TRY((launch_spread2<float, S2_BLOCKS_MANY, false>(b, b->rows, grid, st)));
+    }
+    if (b->any_general_spread) {
+        if (!fp32) SE_TRY((launch_spread2<double, S2_BLOCKS_FP64, true>(b, b->fac, grid, st)));
+        else SE_TRY((launch_spread2<float, S2_BLOCKS_FP64, true>(b, b->fac, grid, st)));
     }
     if (b->any_spread1) {
         if (b->precision == SE_FP32)

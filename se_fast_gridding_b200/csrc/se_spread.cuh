@@ -1,6 +1,7 @@
 // se_spread.cuh -- the spread (SE_FGG_grid, SE_fgg.c:3866-4028) with the
-// periodic fold (SE_FGG_wrap_fcn, SE_fgg.c:327-352) fused, output-stationary.
-// Included inside namespace se by se_solve.cu.
+// periodic fold (SE_FGG_wrap_fcn, SE_fgg.c:327-352) fused, output-stationary, for the grids
+// on which a stencil may cover a cell more than once as seen from one tile (M < P +
+// 15).  Included inside namespace se by se_solve.cu.
 //
 // One CTA owns a TX x TY x TZ tile of one system's periodic grid and visits
 // every particle whose stencil reaches the tile: the particles of at most
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(SPREAD_THREADS, sizeof(Acc) == 4 ? 4 : 2) k_sp
 
     const int tile = blockIdx.x;
     const SysDev& S = sys[find_sys(tile_prefix, nsys, tile)];
-    if (S.path & PATH_TILE_SPREAD) return;   // k_spread2 covers this system
+    if ((S.path & PATH_TILE_SPREAD) || spread2_general(S.path, S.M, S.P)) return;   // k_spread2 covers this system
     const int lt = tile - S.tile_base;
     const int x0 = (lt / (S.nt[1] * S.nt[2])) * TX;
     const int y0 = ((lt / S.nt[2]) % S.nt[1]) * TY;

@@ -1,7 +1,8 @@
 // se_spread2.cuh -- the spread (SE_FGG_grid, SE_fgg.c:3866-4028) with the
 // periodic fold (SE_FGG_wrap_fcn, SE_fgg.c:327-352) fused, for the systems
 // whose grid is cut into whole 16^3 tiles (M a multiple of 16, M >= 32) and
-// whose stencil fits two tiles (P <= 16).  Included inside namespace se by
+// whose stencil fits two tiles (P <= 16), and, on P-wide factor rows (GEN, at
+// the kernel), for all others but the smallest grids.  Included inside namespace se by
 // se_solve.cu after se_spread.cuh (whose bin-range helpers it uses).
 //
 // Factor rows aligned to tiles.  k_factors writes, per particle and axis, a
@@ -48,7 +49,7 @@
 // instructions than the FMAs.)
 //
 // Crowded tiles are split.  Each warp's candidate list is cut into parts of
-// at most S2_CAP candidates; k_tile_parts counts the candidates of each
+// at most S2_CAP candidates (split_cap); k_tile_parts counts the candidates of each
 // tile's most crowded block and scans the part counts, and k_spread2 runs
 // one CTA per part, whose warps take part s of their own lists.  Part 0
 // writes the tile into the grid as above; part s >= 1 writes its sums into
@@ -67,16 +68,27 @@
 #define SE_S2_UNROLL 16
 #endif
 constexpr int S2_CAP = SE_S2_CAP;   // candidates per part of a warp's list
+// ... and of a system of N particles: off the whole tiles, where a particle is a
+// candidate of up to 4^3 or 5^3 tiles, at least N / 512, which bounds its slabs by 2 GB
+__host__ __device__ inline int split_cap(int path, int N)
+{
+    return path & PATH_TILE_SPREAD || N / 512 < S2_CAP ? S2_CAP : N / 512;
+}
 constexpr int S2_WARPS = 4;   // warp blocks per tile
 // warps per CTA: a tile's four warp blocks run as S2_WARPS / CW CTAs (the warps
 // are independent), so that the SMs share out the blocks more evenly: one warp
 // in FP32 (against two: 1M uniform, M = 256, P = 12 0.548 -> 0.529 ms, 256
 // systems of M = 64 2.10 -> 2.05 ms, 16M clustered no difference), two in FP64
 // (2M clustered 2.28 -> 2.23 ms)
-template <typename Acc>
-constexpr int s2_cta_warps() { return sizeof(Acc) == 4 ? 1 : 2; }
+template <typename F, bool GEN>
+constexpr bool s2_fp32_sums() { return sizeof(F) == 4 && !GEN; }
+template <typename F, bool GEN>
+constexpr int s2_cta_warps() { return s2_fp32_sums<F, GEN>() ? 1 : 2; }
 constexpr int S2_LIST = 64;    // per-class list ring: >= group - 1 + 32
-constexpr int S2_SEGS = 64;    // bin segments reaching a warp's block: <= 5 x 4 x 2 for P <= 16
+// bin segments reaching a warp's block: <= 5 x 4 x 2 on whole tiles (P <= 16),
+// <= 8 x 7 x 2 otherwise (P <= 32, the last bin of an axis cut)
+template <bool GEN>
+constexpr int s2_segs() { return GEN ? 112 : 40; }
 constexpr int S2_FOLD = 512;   // FP32 partial sums cover this many of a warp's particles
 // x classes of a particle in a tile: its x row meets both 8-cell halves,
 // the low half only, the high half only
@@ -87,39 +99,53 @@ constexpr int S2_UNROLL = SE_S2_UNROLL;   // particles per unrolled pass of a gr
 // resident at once either way; FP64: 3
 constexpr int S2_BLOCKS_MANY = 5, S2_BLOCKS_FEW = 4, S2_BLOCKS_FP64 = 4;
 
-// particles a warp stages at once: one per lane (FP32), half a warp (FP64)
-template <typename Acc>
-constexpr int s2_group() { return sizeof(Acc) == 4 ? 32 : 16; }
+// particles a warp stages at once: one per lane (FP32 sums), half a warp (FP64)
+template <typename F, bool GEN>
+constexpr int s2_group() { return s2_fp32_sums<F, GEN>() ? 32 : 16; }
 
-template <typename Acc>
+template <typename F, bool GEN>
 struct Spread2Stage {
-    Acc px[s2_group<Acc>()][16];
-    Acc pz[s2_group<Acc>()][8];
-    Acc py[s2_group<Acc>()][8];
-    double q[s2_group<Acc>()];
+    F px[s2_group<F, GEN>()][16];
+    F pz[s2_group<F, GEN>()][8];
+    F py[s2_group<F, GEN>()][8];
+    double q[s2_group<F, GEN>()];
 };
 
 // Where entry x of staged particle k's x row and entry z of its y and z rows
-// lie in the row: in FP64 moved (whole 32-byte groups) so that a warp's operand
-// loads, 8 entries of 4 consecutive particles, fall in distinct banks.
-template <typename Acc>
+// lie in the row: for the matrix instructions moved (whole 32-byte groups) so that
+// a warp's operand loads, 8 entries of 4 consecutive particles, fall in distinct
+// banks.
+template <typename F, bool GEN>
 __device__ __forceinline__ int s2_px(int k, int x)
 {
-    return sizeof(Acc) == 4 ? x : x ^ ((k & 3) << 2);
+    if (sizeof(F) == 4) return GEN ? x ^ (((k >> 1) & 1) << 3) : x;
+    return x ^ ((k & 3) << 2);
 }
 
-template <typename Acc>
+template <typename F>
 __device__ __forceinline__ int s2_pz(int k, int z)
 {
-    return sizeof(Acc) == 4 ? z : z ^ (((k >> 1) & 1) << 2);
+    return sizeof(F) == 4 ? z : z ^ (((k >> 1) & 1) << 2);
 }
 
-template <typename Acc, int CW>
+// A listed particle: 8 particle + 4 hx + 2 hy + hz, the halves of its
+// tile-aligned rows; on the P-wide rows (GEN) the particle and its stencil's
+// entries at the tile's first x and the block's first y and z, plus 16, packed.
+template <bool GEN>
+struct Spread2Entry {
+    using Type = unsigned;
+};
+template <>
+struct Spread2Entry<true> {
+    using Type = uint2;
+};
+
+template <typename F, int CW, bool GEN>
 struct Spread2Smem {
-    Spread2Stage<Acc> stage[CW][2];
-    unsigned list[CW][S2_CLASSES][S2_LIST];   // 8 particle + 4 hx + 2 hy + hz (the halves of its rows)
-    int seg_beg[CW][S2_SEGS];
-    int seg_pre[CW][S2_SEGS];
+    Spread2Stage<F, GEN> stage[CW][2];
+    typename Spread2Entry<GEN>::Type list[CW][S2_CLASSES][S2_LIST];
+    int seg_beg[CW][s2_segs<GEN>()];
+    int seg_pre[CW][s2_segs<GEN>()];
 };
 
 __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc)
@@ -142,6 +168,13 @@ __device__ __forceinline__ void cp_async16_or_zero(void* sdst, const void* gsrc,
                  : "memory");
 }
 
+__device__ __forceinline__ void cp_async_one_or_zero(float* sdst, const float* gsrc, bool on)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(gsrc), "r"(on ? 4 : 0)
+                 : "memory");
+}
+
 __device__ __forceinline__ void cp_async8_or_zero(void* sdst, const void* gsrc, bool on)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
@@ -149,15 +182,21 @@ __device__ __forceinline__ void cp_async8_or_zero(void* sdst, const void* gsrc, 
                  : "memory");
 }
 
+__device__ __forceinline__ void cp_async_one_or_zero(double* sdst, const double* gsrc, bool on)
+{
+    cp_async8_or_zero(sdst, gsrc, on);
+}
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// The 32 cells of one lane: 16 x for z and for z + 1.
+// A warp's sums: 16 x 8 x 8 cells, 32 per lane.
 template <typename Acc>
 struct Spread2Accum;
 
+// FP32: 16 x for z and for z + 1.
 template <>
 struct Spread2Accum<float> {
     float2 a[8], b[8];   // packed x pairs for z and z + 1
@@ -221,6 +260,12 @@ struct Spread2Accum<float> {
     }
 };
 
+// The cells of a block that lie on the grid: x < nx from the lane's first
+// cell on, y < ny and z < nz (nothing outside is stored).
+struct BlockBounds {
+    int nx, ny, nz;
+};
+
 // FP64: the cells of the warp's block as the matrix instructions spread them
 // over a warp: with g = lane / 4 and t = lane % 4, x in {g, g + 8}, every y, z in
 // {2 t, 2 t + 1}.  One instruction adds 4 particles to 8 x by 8 z cells of one y:
@@ -237,17 +282,17 @@ struct Spread2Accum<double> {
     }
     // staged particles i .. i + 3, particle i + t the contraction's element t;
     // HALVES bit 0: x in [0, 8), bit 1: x in [8, 16)
-    template <int HALVES>
-    __device__ __forceinline__ void add(const Spread2Stage<double>& st, int i, int g, int t)
+    template <int HALVES, typename F, bool GEN>
+    __device__ __forceinline__ void add(const Spread2Stage<F, GEN>& st, int i, int g, int t)
     {
         const int k = i + t;
-        const double a0 = (HALVES & 1) ? st.px[k][s2_px<double>(t, g)] : 0.0;
-        const double a1 = (HALVES & 2) ? st.px[k][s2_px<double>(t, g + 8)] : 0.0;
-        const double pz = st.q[k] * st.pz[k][s2_pz<double>(t, g)];
+        const double a0 = (HALVES & 1) ? (double)st.px[k][s2_px<F, GEN>(t, g)] : 0.0;
+        const double a1 = (HALVES & 2) ? (double)st.px[k][s2_px<F, GEN>(t, g + 8)] : 0.0;
+        const double pz = st.q[k] * (double)st.pz[k][s2_pz<F>(t, g)];
 #pragma unroll
         for (int y = 0; y < 8; y += 2) {
-            const double2 py = *reinterpret_cast<const double2*>(&st.py[k][s2_pz<double>(t, y)]);
-            const double b0 = py.x * pz, b1 = py.y * pz;
+            const auto py = *reinterpret_cast<const std::conditional_t<sizeof(F) == 4, float2, double2>*>(&st.py[k][s2_pz<F>(t, y)]);
+            const double b0 = (double)py.x * pz, b1 = (double)py.y * pz;
             if (HALVES & 1) mma_f64(v[y][0], v[y][1], a0, b0);
             if (HALVES & 2) mma_f64(v[y][2], v[y][3], a1, b0);
             if (HALVES & 1) mma_f64(v[y + 1][0], v[y + 1][1], a0, b1);
@@ -255,10 +300,10 @@ struct Spread2Accum<double> {
         }
     }
     // the first n particles of the stage (zero rows up to a multiple of 4)
-    template <int HALVES>
-    __device__ __forceinline__ void add_group(const Spread2Stage<double>& st, int n, int g, int t)
+    template <int HALVES, typename F, bool GEN>
+    __device__ __forceinline__ void add_group(const Spread2Stage<F, GEN>& st, int n, int g, int t)
     {
-        constexpr int G = s2_group<double>();
+        constexpr int G = s2_group<F, GEN>();
         if (n == G) {
 #pragma unroll
             for (int i = 0; i < G; i += 4) add<HALVES>(st, i, g, t);
@@ -277,6 +322,19 @@ struct Spread2Accum<double> {
             for (int y = 0; y < 8; y++)
                 *reinterpret_cast<double2*>(cell0 + 8 * h * plane + y * row) =
                     make_double2(v[y][2 * h], v[y][2 * h + 1]);
+    }
+    // the same on a grid that may end inside the block (its rows of any alignment)
+    __device__ __forceinline__ void store(double* cell0, long long plane, int row, const BlockBounds& in) const
+    {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int y = 0; y < 8; y++) {
+                double* c = cell0 + 8 * h * plane + y * row;
+                if (8 * h >= in.nx || y >= in.ny) continue;
+                if (in.nz > 0) c[0] = v[y][2 * h];
+                if (in.nz > 1) c[1] = v[y][2 * h + 1];
+            }
     }
 };
 
@@ -318,6 +376,7 @@ __device__ __forceinline__ int block_candidates(const SysDev& S, int lt, int w,
 {
     const int nt = S.nt[0];
     const int tix = lt / (nt * nt), tiy = (lt / nt) % nt, tiz = lt % nt;
+    if (tiy * 16 + 8 * (w >> 1) >= S.M || tiz * 16 + 8 * (w & 1) >= S.M) return 0;
     const BlockBins B(S, tix * 16, tiy * 16 + 8 * (w >> 1), tiz * 16 + 8 * (w & 1));
     int sum = 0;
     for (int u = lane; u < B.segments(); u += 32) {
@@ -331,12 +390,12 @@ __device__ __forceinline__ int block_candidates(const SysDev& S, int lt, int w,
 }
 
 // Parts per tile (one warp per warp block, two tiles per CTA:
-// max(1, ceil(candidates of the most crowded block / S2_CAP)) for the
+// max(1, ceil(candidates of the most crowded block / split_cap)) for the
 // k_spread2 systems, 1 for the others), then, in the block that finishes
 // last, their exclusive scan in place: parts[t] = the first part of tile t,
-// parts[ntiles] = the number of parts, and part_tile[s] = the tile of part s.  More parts than the launch bound
-// (which no input reaches: a bin is a candidate of at most two tiles per
-// axis) set bit 2 of err.  The block counter is left at zero for the next
+// parts[ntiles] = the number of parts, and part_tile[s] = the tile of part s.
+// More parts than the launch bound (which no input reaches: split_slots) set
+// bit 2 of err.  The block counter is left at zero for the next
 // launch.
 constexpr int TP_WARPS = 8;
 constexpr int TP_TILES = TP_WARPS / S2_WARPS;   // tiles per CTA
@@ -349,10 +408,12 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x * TP_TILES + warp / S2_WARPS, wb = warp % S2_WARPS;
     __shared__ int cand[TP_WARPS];
-    int c = 0;
+    int c = 0, cap = S2_CAP;
     if (tile < ntiles) {
         const SysDev& S = sys[find_sys(tile_prefix, nsys, tile)];
-        if (S.path & PATH_TILE_SPREAD) c = block_candidates(S, tile - S.tile_base, wb, boff, lane);
+        cap = split_cap(S.path, S.N);
+        if ((S.path & PATH_TILE_SPREAD) || spread2_general(S.path, S.M, S.P))
+            c = block_candidates(S, tile - S.tile_base, wb, boff, lane);
     }
     if (lane == 0) cand[warp] = c;
     __syncthreads();
@@ -360,7 +421,7 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
         int most = 0;
 #pragma unroll
         for (int k = 0; k < S2_WARPS; k++) most = max(most, cand[warp + k]);
-        parts[tile] = max(1, (most + S2_CAP - 1) / S2_CAP);
+        parts[tile] = max(1, (most + cap - 1) / cap);
     }
     __shared__ int last;
     __shared__ int wsum[TP_WARPS];
@@ -415,39 +476,54 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
     }
 }
 
-// CW warps per CTA (S2_WARPS / CW CTAs per part of a tile)
-template <typename Acc, int BLOCKS, int CW = s2_cta_warps<Acc>()>
+// CW warps per CTA (S2_WARPS / CW CTAs per part of a tile); tile_parts null: no
+// tile has a second part.  GEN: the systems of spread2_general, with rows the
+// P-wide factor rows (PS entries apart), copied one entry at a time, tiles that may
+// reach past the grid's end, and FP64 sums of FP32 factors too: as fast there as
+// FP32 sums (58,600 particles, M = 100, P = 12: 0.115 ms both) and closer (a
+// third of the error or less).  Against k_spread, which builds each chunk's rows
+// per CTA, B200, FP64 spread stage: 58,600 particles, M = 100, P = 8 0.142 ->
+// 0.069 ms, P = 12 0.292 -> 0.110, P = 24 0.837 -> 0.379; 3,900, P = 8 0.023 ->
+// 0.016; 122,000, M = 250, P = 12 0.483 -> 0.183; 41,000, M = 128, P = 21 0.391 ->
+// 0.142.  FP32 0.131 -> 0.071, 0.238 -> 0.115, 0.627 -> 0.396, 0.021 -> 0.016,
+// 0.265 -> 0.185, 0.215 -> 0.146.  (45 particles, M = 36: 0.012 -> 0.013.)
+template <typename F, int BLOCKS, bool GEN = false, int CW = s2_cta_warps<F, GEN>()>
 __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     const SysDev* __restrict__ sys, const int* __restrict__ tile_sys,
     const double4* __restrict__ srec, const int* __restrict__ sg,
-    const Acc* __restrict__ rows, const int* __restrict__ boff, double* __restrict__ grid,
+    const F* __restrict__ rows, int PS, const int* __restrict__ boff, double* __restrict__ grid,
     const int* __restrict__ tile_parts, const int* __restrict__ part_tile, int ntiles,
     int* __restrict__ tile_done, double* __restrict__ slab, int slab_slots,
     int* __restrict__ err)
 {
-    constexpr bool FOLD = sizeof(Acc) == 4;
-    constexpr int G = s2_group<Acc>();
-    constexpr int V = 16 / sizeof(Acc);   // entries per 16-byte copy
+    constexpr bool FOLD = s2_fp32_sums<F, GEN>();
+    using Acc = std::conditional_t<FOLD, float, double>;
+    constexpr int G = s2_group<F, GEN>();
+    constexpr int V = 16 / sizeof(F);   // entries per 16-byte copy
     constexpr int S2_CTA_SPLIT = S2_WARPS / CW, S2_THREADS = CW * 32;
-    __shared__ __align__(16) Spread2Smem<Acc, CW> sm;
+    __shared__ __align__(16) Spread2Smem<F, CW, GEN> sm;
     __shared__ int folds;   // this CTA finished its tile's parts last
 
     // ---- the part this CTA sums and its tile (k_tile_parts' part_tile; warp
     // blocks sub CW + [0, CW) of it), and the tile's system
     const int item = blockIdx.x / S2_CTA_SPLIT, sub = blockIdx.x % S2_CTA_SPLIT;
-    const int nall = tile_parts[ntiles];
-    const int tile = part_tile[item];   // (the grid holds at most `bound` parts)
-    if (item >= nall) return;
+    int tile = item;
+    if (tile_parts) {
+        const int nall = tile_parts[ntiles];
+        tile = part_tile[item];   // (the grid holds at most `bound` parts)
+        if (item >= nall) return;
+    }
     if ((unsigned)tile >= (unsigned)ntiles) {   // cannot happen: flagged, nothing summed
         if (threadIdx.x == 0) atomicOr(err, 2);
         return;
     }
-    const int first = tile_parts[tile];
+    const int first = tile_parts ? tile_parts[tile] : tile;
     const int ipart = item - first;
-    const int nparts = tile_parts[tile + 1] - first;
+    const int nparts = tile_parts ? tile_parts[tile + 1] - first : 1;
     const SysDev& S = sys[tile_sys[tile]];
-    if (!(S.path & PATH_TILE_SPREAD)) return;   // k_spread covers this system
-    const int slot0 = tile_parts[tile] - tile;   // slab slot of part 1
+    // the other variant or k_spread covers the other systems
+    if (!(GEN ? spread2_general(S.path, S.M, S.P) : (S.path & PATH_TILE_SPREAD) != 0)) return;
+    const int slot0 = first - tile;   // slab slot of part 1
     if (ipart > 0 && slot0 + ipart - 1 >= slab_slots) {   // cannot happen: see k_tile_parts
         if (threadIdx.x == 0) atomicOr(err, 2);
         return;
@@ -463,9 +539,10 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
 
     // ---- the bin segments reaching this warp's block (at most 5 x 4 x 2) and
     // their prefix: the warp's own candidate list, in segment order
-    const BlockBins B(S, x0, y0 + 8 * wy, z0 + 8 * wz);
-    int nseg = B.segments();
-    if (nseg > S2_SEGS) {   // cannot happen for M >= 32 and P <= 16: flagged, the block sums nothing
+    const bool outside = GEN && (y0 + 8 * wy >= M || z0 + 8 * wz >= M);   // no cell of the block is on the grid
+    const BlockBins B(S, x0, outside ? 0 : y0 + 8 * wy, outside ? 0 : z0 + 8 * wz);
+    int nseg = outside ? 0 : B.segments();
+    if (nseg > s2_segs<GEN>()) {   // cannot happen: flagged, the block sums nothing
         if (lane == 0) atomicOr(err, 2);
         nseg = 0;
     }
@@ -501,7 +578,8 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
                                 : slab + (long long)(slot0 + ipart - 1) * 4096) +
                     (long long)(8 * wy) * row + 8 * wz + lz + (FOLD ? (long long)ly * row : ly * plane);
     // this part's candidates: [cbeg, cend) of the warp's list
-    const int cbeg = ipart * S2_CAP, cend = min(total, cbeg + S2_CAP);
+    const int cap = GEN ? split_cap(S.path, S.N) : S2_CAP;   // (ipart cap < N + cap)
+    const int cbeg = ipart * cap, cend = min(total, cbeg + cap);
 
     Spread2Accum<Acc> acc;
     acc.zero();
@@ -532,21 +610,37 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
         // candidate is listed), each class in candidate order
         while (!(cnt & FULL) && cpos < cend) {
             int cls = -1;
-            unsigned entry = 0;
+            typename Spread2Entry<GEN>::Type entry = {};
             if (cpos + lane < cend) {
-                // per axis: which tile after the home tile this one is, and
-                // the stencil's entry at the tile's (block's) first cell
-                int hx = tix - (g_of(pk, 0) >> 4), hy = tiy - (g_of(pk, 1) >> 4), hz = tiz - (g_of(pk, 2) >> 4);
-                hx += hx < 0 ? nt : 0;
-                hy += hy < 0 ? nt : 0;
-                hz += hz < 0 ? nt : 0;
-                const int ex = 16 * hx - (g_of(pk, 0) & 15);
-                const int ey = 16 * hy - (g_of(pk, 1) & 15) + 8 * wy, ez = 16 * hz - (g_of(pk, 2) & 15) + 8 * wz;
                 // 8 cells from entry e on meet the stencil's entries [0, P)
                 auto meets = [&](int e) { return (unsigned)(e + 7) < (unsigned)(P + 7); };
-                const bool lo = meets(ex), hi = meets(ex + 8);
-                if (meets(ey) && meets(ez)) cls = lo ? (hi ? 0 : 1) : (hi ? 2 : -1);
-                entry = ((unsigned)part << 3) | (hx << 2) | (hy << 1) | hz;
+                bool lo, hi, yz;
+                if constexpr (GEN) {
+                    // the stencil's entry at the tile's (block's) first cell: the
+                    // corner lies in the tile or less than M - 15 before it
+                    int ex = x0 - g_of(pk, 0), ey = y0 + 8 * wy - g_of(pk, 1), ez = z0 + 8 * wz - g_of(pk, 2);
+                    ex += ex < -15 ? M : 0;
+                    ey += ey < -7 ? M : 0;
+                    ez += ez < -7 ? M : 0;
+                    lo = meets(ex);
+                    hi = meets(ex + 8);
+                    yz = meets(ey) && meets(ez);
+                    entry = make_uint2((unsigned)part, (unsigned)((ex + 16) | (ey + 16) << 10 | (ez + 16) << 20));
+                } else {
+                    // per axis: which tile after the home tile this one is, and
+                    // the stencil's entry at the tile's (block's) first cell
+                    int hx = tix - (g_of(pk, 0) >> 4), hy = tiy - (g_of(pk, 1) >> 4), hz = tiz - (g_of(pk, 2) >> 4);
+                    hx += hx < 0 ? nt : 0;
+                    hy += hy < 0 ? nt : 0;
+                    hz += hz < 0 ? nt : 0;
+                    const int ex = 16 * hx - (g_of(pk, 0) & 15);
+                    const int ey = 16 * hy - (g_of(pk, 1) & 15) + 8 * wy, ez = 16 * hz - (g_of(pk, 2) & 15) + 8 * wz;
+                    lo = meets(ex);
+                    hi = meets(ex + 8);
+                    yz = meets(ey) && meets(ez);
+                    entry = ((unsigned)part << 3) | (hx << 2) | (hy << 1) | hz;
+                }
+                if (yz) cls = lo ? (hi ? 0 : 1) : (hi ? 2 : -1);
             }
             const unsigned k0 = __ballot_sync(0xffffffffu, cls == 0);
             const unsigned k1 = __ballot_sync(0xffffffffu, cls == 1);
@@ -569,36 +663,64 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
         const int sh = 8 * cls;
         const int avail = (cnt >> sh) & 0xFF;
         const int head = (ring >> sh) & (S2_LIST - 1);
-        const unsigned* list = sm.list[lw][cls];
+        const auto* list = sm.list[lw][cls];
         // ---- stage the next group of the class: the x tile rows (of a
         // one-half class, that half), the block's 8 y and 8 z entries and the
         // charges, zeros past the group's n particles; consecutive lanes copy
         // consecutive 16-byte pieces of a row
         const int n = min(G, avail);
         if (n > 0) {
-            Spread2Stage<Acc>& st = sm.stage[lw][buf];
-            constexpr int C8 = 8 / V, C16 = 16 / V;   // pieces per 8 and 16 entries
-            if (cls == 0) {
+            Spread2Stage<F, GEN>& st = sm.stage[lw][buf];
+            if constexpr (GEN) {
+                // entry by entry, zeros outside the stencil
+                auto copy = [&](F* dst, int i, int a, int k) {
+                    const uint2 e = i < n ? list[(head + i) & (S2_LIST - 1)] : make_uint2(0u, 0u);
+                    const int j = (int)(e.y >> (10 * a) & 1023u) - 16 + k;
+                    const bool on = i < n && (unsigned)j < (unsigned)P;
+                    cp_async_one_or_zero(dst, rows + ((long long)e.x * 3 + a) * PS + (on ? j : 0), on);
+                };
+                if (cls == 0) {
+#pragma unroll 4
+                    for (int i = lane >> 4; i < G; i += 2)
+                        copy(&st.px[i][s2_px<F, GEN>(i, lane & 15)], i, 0, lane & 15);
+                } else {
+                    const int k = 8 * (cls - 1) + (lane & 7);
+#pragma unroll 4
+                    for (int i = lane >> 3; i < G; i += 4) copy(&st.px[i][s2_px<F, GEN>(i, k)], i, 0, k);
+                }
+#pragma unroll 4
+                for (int i = lane >> 3; i < G; i += 4) {
+                    copy(&st.py[i][s2_pz<F>(i, lane & 7)], i, 1, lane & 7);
+                    copy(&st.pz[i][s2_pz<F>(i, lane & 7)], i, 2, lane & 7);
+                }
+                if (lane < G) {
+                    const unsigned p = lane < n ? list[(head + lane) & (S2_LIST - 1)].x : 0u;
+                    cp_async8_or_zero(&st.q[lane], &srec[p].w, lane < n);
+                }
+            } else {
+                constexpr int C8 = 8 / V, C16 = 16 / V;   // pieces per 8 and 16 entries
+                if (cls == 0) {
 #pragma unroll
-                for (int i0 = 0; i0 < G; i0 += 32 / C16) {
-                    const int i = i0 + lane / C16, k = V * (lane % C16);
+                    for (int i0 = 0; i0 < G; i0 += 32 / C16) {
+                        const int i = i0 + lane / C16, k = V * (lane % C16);
+                        const unsigned e = i < n ? list[(head + i) & (S2_LIST - 1)] : 0u;
+                        cp_async16_or_zero(&st.px[i][s2_px<F, GEN>(i, k)],
+                                           rows + (long long)(e >> 3) * 96 + 4 * (e & 4) + k, i < n);
+                    }
+                }
+#pragma unroll
+                for (int i0 = 0; i0 < G; i0 += 32 / C8) {
+                    const int i = i0 + lane / C8, k = V * (lane % C8);
                     const unsigned e = i < n ? list[(head + i) & (S2_LIST - 1)] : 0u;
-                    cp_async16_or_zero(&st.px[i][s2_px<Acc>(i, k)],
-                                       rows + (long long)(e >> 3) * 96 + 4 * (e & 4) + k, i < n);
+                    const Acc* r = rows + (long long)(e >> 3) * 96 + k;
+                    if (cls != 0) {
+                        const int o = 8 * (cls - 1);
+                        cp_async16_or_zero(&st.px[i][s2_px<F, GEN>(i, o + k)], r + 4 * (e & 4) + o, i < n);
+                    }
+                    cp_async16_or_zero(&st.py[i][s2_pz<F>(i, k)], r + 32 + 8 * (e & 2) + 8 * wy, i < n);
+                    cp_async16_or_zero(&st.pz[i][s2_pz<F>(i, k)], r + 64 + 16 * (e & 1) + 8 * wz, i < n);
+                    if (k == 0) cp_async8_or_zero(&st.q[i], &srec[e >> 3].w, i < n);
                 }
-            }
-#pragma unroll
-            for (int i0 = 0; i0 < G; i0 += 32 / C8) {
-                const int i = i0 + lane / C8, k = V * (lane % C8);
-                const unsigned e = i < n ? list[(head + i) & (S2_LIST - 1)] : 0u;
-                const Acc* r = rows + (long long)(e >> 3) * 96 + k;
-                if (cls != 0) {
-                    const int o = 8 * (cls - 1);
-                    cp_async16_or_zero(&st.px[i][s2_px<Acc>(i, o + k)], r + 4 * (e & 4) + o, i < n);
-                }
-                cp_async16_or_zero(&st.py[i][s2_pz<Acc>(i, k)], r + 32 + 8 * (e & 2) + 8 * wy, i < n);
-                cp_async16_or_zero(&st.pz[i][s2_pz<Acc>(i, k)], r + 64 + 16 * (e & 1) + 8 * wz, i < n);
-                if (k == 0) cp_async8_or_zero(&st.q[i], &srec[e >> 3].w, i < n);
             }
             cp_async_commit();
             cnt -= (unsigned)n << sh;
@@ -610,7 +732,7 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
             if (n > 0) cp_async_wait<1>();
             else cp_async_wait<0>();
             __syncwarp();
-            Spread2Stage<Acc>& st = sm.stage[lw][buf ^ 1];
+            Spread2Stage<F, GEN>& st = sm.stage[lw][buf ^ 1];
             if constexpr (FOLD) {
                 // lane i scales its particle's 8 y entries by the charge, once
                 if (lane < pending) {
@@ -666,6 +788,10 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     // ---- the lane's cells
     if constexpr (FOLD) {
         if (since_fold > 0 || !written) acc.fold(cell0, plane, !written);
+    } else if (GEN) {
+        // (a slab holds whole tiles)
+        const int end = ipart == 0 ? M : nt * 16;
+        acc.store(cell0, plane, row, {end - x0 - ly, end - y0 - 8 * wy, end - z0 - 8 * wz - lz});
     } else {
         acc.store(cell0, plane, row);
     }
@@ -681,6 +807,7 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
             __threadfence();
             for (int c = t; c < 4096; c += S2_THREADS) {
                 const int x = c >> 8, y = (c >> 4) & 15, z = c & 15;
+                if (GEN && (x0 + x >= M || y0 + y >= M || z0 + z >= M)) continue;
                 double* gp = gs + (long long)(x0 + x) * gplane + (long long)(y0 + y) * M + z0 + z;
                 double v = __ldcg(gp);
                 for (int k = 0; k < nparts - 1; k++)
