@@ -50,11 +50,11 @@ constexpr int PATH_FFT3 = 16;          // the batch's FP64 FFTs through se_fft.c
 constexpr int PATH_BIN_WINDOWS = 32;   // k_interp2 stages one window per bin (not per z pair)
 
 // Whether a system off the whole tiles spreads by k_spread2 on its P-wide
-// factor rows: where no cell lies in a stencil twice as seen from one 16^3 tile
-// (M >= P + 15); k_spread serves the smaller grids.
+// factor rows: where a run of 8 cells meets a stencil in one piece (M >= P + 7);
+// k_spread serves the smaller grids.
 __host__ __device__ inline bool spread2_general(int path, int M, int P)
 {
-    return !(path & PATH_TILE_SPREAD) && M >= P + 15;
+    return !(path & PATH_TILE_SPREAD) && M >= P + 7;
 }
 
 // Whether k_interp3 serves a system (else k_interp2 on the path with

@@ -14,7 +14,7 @@
 //               (tile-aligned rows for the tile kernels)
 //   spread      k_tile_parts + k_spread2, one CTA per part of a 16^3 tile,
 //               the fold fused (se_spread2.cuh); k_spread (se_spread.cuh) on
-//               the smallest grids (M < P + 15)
+//               the smallest grids (M < P + 7)
 //   cuFFT D2Z, k_scale (Z of scaling(), SE_general.c:145-175, applied to the
 //               half spectrum as product_rc does, SE_general.c:336-362), Z2D
 //   interp      one launch per stencil and mode of the batch, the unfold fused:

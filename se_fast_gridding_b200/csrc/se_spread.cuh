@@ -1,7 +1,7 @@
 // se_spread.cuh -- the spread (SE_FGG_grid, SE_fgg.c:3866-4028) with the
-// periodic fold (SE_FGG_wrap_fcn, SE_fgg.c:327-352) fused, output-stationary, for the grids
-// on which a stencil may cover a cell more than once as seen from one tile (M < P +
-// 15).  Included inside namespace se by se_solve.cu.
+// periodic fold (SE_FGG_wrap_fcn, SE_fgg.c:327-352) fused, output-stationary,
+// for grids so small that 8 cells may meet a stencil in two pieces (M < P + 7).
+// Included inside namespace se by se_solve.cu.
 //
 // One CTA owns a TX x TY x TZ tile of one system's periodic grid and visits
 // every particle whose stencil reaches the tile: the particles of at most

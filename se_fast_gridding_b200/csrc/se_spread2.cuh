@@ -130,7 +130,8 @@ __device__ __forceinline__ int s2_pz(int k, int z)
 
 // A listed particle: 8 particle + 4 hx + 2 hy + hz, the halves of its
 // tile-aligned rows; on the P-wide rows (GEN) the particle and its stencil's
-// entries at the tile's first x and the block's first y and z, plus 16, packed.
+// entries at the first x of both 8-cell halves and the block's first y and z, plus
+// 8, a byte each.
 template <bool GEN>
 struct Spread2Entry {
     using Type = unsigned;
@@ -486,7 +487,8 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
 // 0.069 ms, P = 12 0.292 -> 0.110, P = 24 0.837 -> 0.379; 3,900, P = 8 0.023 ->
 // 0.016; 122,000, M = 250, P = 12 0.483 -> 0.183; 41,000, M = 128, P = 21 0.391 ->
 // 0.142.  FP32 0.131 -> 0.071, 0.238 -> 0.115, 0.627 -> 0.396, 0.021 -> 0.016,
-// 0.265 -> 0.185, 0.215 -> 0.146.  (45 particles, M = 36: 0.012 -> 0.013.)
+// 0.265 -> 0.185, 0.215 -> 0.146.  45 particles, M = 36:
+// 0.012 -> 0.013.  5,100, M = 32, P = 21 FP64 0.770 -> 0.467.
 template <typename F, int BLOCKS, bool GEN = false, int CW = s2_cta_warps<F, GEN>()>
 __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     const SysDev* __restrict__ sys, const int* __restrict__ tile_sys,
@@ -616,16 +618,20 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
                 auto meets = [&](int e) { return (unsigned)(e + 7) < (unsigned)(P + 7); };
                 bool lo, hi, yz;
                 if constexpr (GEN) {
-                    // the stencil's entry at the tile's (block's) first cell: the
-                    // corner lies in the tile or less than M - 15 before it
-                    int ex = x0 - g_of(pk, 0), ey = y0 + 8 * wy - g_of(pk, 1), ez = z0 + 8 * wz - g_of(pk, 2);
-                    ex += ex < -15 ? M : 0;
-                    ey += ey < -7 ? M : 0;
-                    ez += ez < -7 ? M : 0;
-                    lo = meets(ex);
-                    hi = meets(ex + 8);
+                    // the stencil's entry at the first cell of 8: the corner lies
+                    // among them or less than M - 7 before them
+                    auto entry_at = [&](int first, int axis) {
+                        const int e = first - g_of(pk, axis);
+                        return e < -7 ? e + M : e;
+                    };
+                    const int el = entry_at(x0, 0), eh = entry_at(x0 + 8, 0);
+                    const int ey = entry_at(y0 + 8 * wy, 1), ez = entry_at(z0 + 8 * wz, 2);
+                    lo = meets(el);
+                    hi = meets(eh);
                     yz = meets(ey) && meets(ez);
-                    entry = make_uint2((unsigned)part, (unsigned)((ex + 16) | (ey + 16) << 10 | (ez + 16) << 20));
+                    // (an entry that meets nothing is not used, or >= P in its byte)
+                    const auto byte = [](int e) { return (unsigned)min(e + 8, 255); };
+                    entry = make_uint2((unsigned)part, byte(el) | byte(eh) << 8 | byte(ey) << 16 | byte(ez) << 24);
                 } else {
                     // per axis: which tile after the home tile this one is, and
                     // the stencil's entry at the tile's (block's) first cell
@@ -673,25 +679,25 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
             Spread2Stage<F, GEN>& st = sm.stage[lw][buf];
             if constexpr (GEN) {
                 // entry by entry, zeros outside the stencil
-                auto copy = [&](F* dst, int i, int a, int k) {
+                auto copy = [&](F* dst, int i, int a, int k, int shift) {
                     const uint2 e = i < n ? list[(head + i) & (S2_LIST - 1)] : make_uint2(0u, 0u);
-                    const int j = (int)(e.y >> (10 * a) & 1023u) - 16 + k;
+                    const int j = (int)(e.y >> shift & 255u) - 8 + k;
                     const bool on = i < n && (unsigned)j < (unsigned)P;
                     cp_async_one_or_zero(dst, rows + ((long long)e.x * 3 + a) * PS + (on ? j : 0), on);
                 };
                 if (cls == 0) {
 #pragma unroll 4
                     for (int i = lane >> 4; i < G; i += 2)
-                        copy(&st.px[i][s2_px<F, GEN>(i, lane & 15)], i, 0, lane & 15);
+                        copy(&st.px[i][s2_px<F, GEN>(i, lane & 15)], i, 0, lane & 7, lane & 8);
                 } else {
                     const int k = 8 * (cls - 1) + (lane & 7);
 #pragma unroll 4
-                    for (int i = lane >> 3; i < G; i += 4) copy(&st.px[i][s2_px<F, GEN>(i, k)], i, 0, k);
+                    for (int i = lane >> 3; i < G; i += 4) copy(&st.px[i][s2_px<F, GEN>(i, k)], i, 0, lane & 7, 8 * (cls - 1));
                 }
 #pragma unroll 4
                 for (int i = lane >> 3; i < G; i += 4) {
-                    copy(&st.py[i][s2_pz<F>(i, lane & 7)], i, 1, lane & 7);
-                    copy(&st.pz[i][s2_pz<F>(i, lane & 7)], i, 2, lane & 7);
+                    copy(&st.py[i][s2_pz<F>(i, lane & 7)], i, 1, lane & 7, 16);
+                    copy(&st.pz[i][s2_pz<F>(i, lane & 7)], i, 2, lane & 7, 24);
                 }
                 if (lane < G) {
                     const unsigned p = lane < n ? list[(head + lane) & (S2_LIST - 1)].x : 0u;
