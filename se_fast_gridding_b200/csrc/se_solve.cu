@@ -566,9 +566,10 @@ static int path_of(const se_system* sys, const int* paths, int i)
 // whole tiles, else with a cut tile of one cell among them.
 static long long split_slots(const se_system& s, int path)
 {
-    if (s.N <= S2_CAP || (!(path & PATH_TILE_SPREAD) && !spread2_general(path, s.M, s.P))) return 0;
+    const int cap = split_cap(path, s.M, s.P, s.N);
+    if (s.N <= cap || (!(path & PATH_TILE_SPREAD) && !spread2_general(path, s.M, s.P))) return 0;
     const long long t = path & PATH_TILE_SPREAD ? 2 : (FB + s.P - 4) / TX + 3;
-    return t * t * t * s.N / split_cap(path, s.N);
+    return t * t * t * s.N / cap;
 }
 
 static size_t batch_bytes(const se_system* sys, int nsys, int precision, int* nbins_out,
@@ -990,7 +991,7 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
         if (path & PATH_TILE_SPREAD) b->any_tile_spread = true;
         else if (spread2_general(path, systems[i].M, systems[i].P)) b->any_general_spread = true;
         else b->any_spread1 = true;
-        if (systems[i].N > S2_CAP) b->split = true;
+        if (systems[i].N > split_cap(path, systems[i].M, systems[i].P, systems[i].N)) b->split = true;
         if (path & PATH_PAIR_INTERP) b->any_interp2 = true;
         else if (const SysDev& S = b->host_sys[i]; !interp3_better(path, precision, S.M, S.P, S.mode)) {
             b->interp_P = !b->any_interp1 || b->interp_P == S.P ? S.P : 0;
@@ -1203,7 +1204,7 @@ static int run_spread(se_batch b, double* grid, cudaStream_t st)
         // the parts of each tile and each part's tile, then one CTA per part
         // (at most the bound; the CTAs past the number of parts return at once).
         // A tile has no more candidates than its system has particles: with at
-        // most S2_CAP each there is nothing to split and no need of the count
+        // most a part's each there is nothing to split and no need of the count
         // (0.009 ms of a spread: 3,900 particles, M = 100, P = 8 0.025 -> 0.016 ms)
         const int bound = b->ntiles + b->slab_slots;
         k_tile_parts<<<ceil_div(b->ntiles, TP_TILES), TP_WARPS * 32, 0, st>>>(

@@ -17,7 +17,8 @@ TOL = {"fp64": 1e-12, "fp32": 2e-6}
                                             (400, 31, 16, 0), (400, 30, 16, 0), (500, 33, 16, 0), (700, 47, 32, 0),
                                             (700, 46, 32, 0), (900, 48, 24, 0), (600, 49, 17, 0), (800, 57, 12, 0),
                                             (100, 8, 1, 0), (200, 19, 12, 0), (200, 18, 12, 0),
-                                            (300, 27, 20, 0), (9000, 32, 21, 1), (500, 39, 32, 0),
+                                            (300, 27, 20, 0), (9000, 32, 21, 1), (5000, 32, 20, 0), (1024, 31, 16, 0),
+                                            (1025, 31, 16, 0), (500, 39, 32, 0),
                                             (400, 38, 32, 0), (20000, 41, 4, 0), (30000, 65, 10, 1), (30000, 50, 9, 1),
                                             (30000, 64, 18, 1)])
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
