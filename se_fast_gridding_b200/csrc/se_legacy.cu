@@ -27,6 +27,7 @@
 
 #include "se_fgg_gpu.h"
 #include "se_internal.h"
+#include "se_mirror_pool.h"
 
 namespace se {
 namespace legacy {
@@ -72,56 +73,18 @@ static bool on_device(const void* p)
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// Device buffers that stand in for the caller's host arrays during a call.
-// A call takes them from this pool and gives them back when it returns (its
-// outputs are in host memory by then), so a caller that passes new host
-// arrays on every call -- spectral_ewald() mallocs its grids per solve --
-// reuses the same device memory instead of allocating it again.  Idle
-// buffers beyond LIMIT bytes are freed, largest first.
-struct MirrorPool {
-    std::mutex mu;
-    std::multimap<size_t, void*> idle;   // capacity -> buffer
-    size_t idle_bytes = 0;
-    static constexpr size_t LIMIT = size_t(16) << 30;
-
-    int acquire(size_t bytes, void** d, size_t* cap)
+struct DeviceBuffers {
+    static int alloc(void** p, size_t bytes)
     {
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            auto it = idle.lower_bound(bytes);
-            if (it != idle.end() && it->first <= 2 * bytes) {   // best fit, at most 2x
-                *d = it->second;
-                *cap = it->first;
-                idle_bytes -= it->first;
-                idle.erase(it);
-                return SE_OK;
-            }
-        }
-        void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(mirror)", __FILE__, __LINE__);
-        *d = p;
-        *cap = bytes;
-        return SE_OK;
+        const cudaError_t e = cudaMalloc(p, bytes);
+        return e == cudaSuccess ? SE_OK : cuda_fail(e, "cudaMalloc(mirror)", __FILE__, __LINE__);
     }
-
-    void release(void* d, size_t cap)
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        idle.emplace(cap, d);
-        idle_bytes += cap;
-        while (idle_bytes > LIMIT && !idle.empty()) {
-            auto it = std::prev(idle.end());
-            cudaFree(it->second);
-            idle_bytes -= it->first;
-            idle.erase(it);
-        }
-    }
+    static void free(void* p) { cudaFree(p); }
 };
 
-static MirrorPool& mirrors()
+static MirrorPool<DeviceBuffers>& mirrors()
 {
-    static MirrorPool* c = new MirrorPool();
+    static auto* c = new MirrorPool<DeviceBuffers>(size_t(16) << 30);
     return *c;
 }
 
@@ -131,21 +94,24 @@ static MirrorPool& mirrors()
 // one mirror.
 class Stager {
 public:
-    Stager() = default;
+    Stager()
+    {
+        if (cudaGetDevice(&dev_) != cudaSuccess) cudaGetLastError();   // (the first use fails)
+    }
     Stager(const Stager&) = delete;
     Stager& operator=(const Stager&) = delete;
     ~Stager()
     {
         for (auto& e : ents_)
-            if (e.host && e.d) mirrors().release(e.d, e.cap);
-        for (auto& b : scratch_) mirrors().release(b.second, b.first);
+            if (e.host && e.d) mirrors().release(dev_, e.d, e.cap);
+        for (auto& b : scratch_) mirrors().release(dev_, b.second, b.first);
     }
     // device memory for the duration of the call, from the same pool
     void* scratch(size_t bytes)
     {
         void* d = nullptr;
         size_t cap = 0;
-        if (err_ || (err_ = mirrors().acquire(bytes, &d, &cap))) return nullptr;
+        if (err_ || (err_ = mirrors().acquire(dev_, bytes, &d, &cap))) return nullptr;
         scratch_.emplace_back(cap, d);
         return d;
     }
@@ -157,9 +123,9 @@ public:
                 if (bytes > e.bytes) {   // grow: take a larger mirror
                     e.bytes = bytes;
                     if (e.host && bytes > e.cap) {
-                        mirrors().release(e.d, e.cap);
+                        mirrors().release(dev_, e.d, e.cap);
                         e.d = nullptr;
-                        if ((err_ = mirrors().acquire(bytes, &e.d, &e.cap))) return nullptr;
+                        if ((err_ = mirrors().acquire(dev_, bytes, &e.d, &e.cap))) return nullptr;
                     }
                 }
                 e.in |= in;
@@ -168,7 +134,7 @@ public:
             }
         Ent e{h, nullptr, bytes, 0, !on_device(h), in, out};
         if (e.host) {
-            if ((err_ = mirrors().acquire(bytes, &e.d, &e.cap))) return nullptr;
+            if ((err_ = mirrors().acquire(dev_, bytes, &e.d, &e.cap))) return nullptr;
         } else {
             e.d = const_cast<void*>(h);
         }
@@ -188,6 +154,7 @@ private:
     };
     std::vector<Ent> ents_;
     std::vector<std::pair<size_t, void*>> scratch_;
+    int dev_ = 0;   // the current device: the mirrors' and the kernels'
     int err_ = 0;
 };
 
