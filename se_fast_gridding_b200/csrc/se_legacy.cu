@@ -74,10 +74,12 @@ static bool on_device(const void* p)
 }
 
 struct DeviceBuffers {
+    // (a failure is left to the caller to report: scratch has a fallback)
     static int alloc(void** p, size_t bytes)
     {
         const cudaError_t e = cudaMalloc(p, bytes);
-        return e == cudaSuccess ? SE_OK : cuda_fail(e, "cudaMalloc(mirror)", __FILE__, __LINE__);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e;
     }
     static void free(void* p) { cudaFree(p); }
 };
@@ -106,12 +108,13 @@ public:
             if (e.host && e.d) mirrors().release(dev_, e.d, e.cap);
         for (auto& b : scratch_) mirrors().release(dev_, b.second, b.first);
     }
-    // device memory for the duration of the call, from the same pool
+    // device memory for the duration of the call, from the same pool; null when
+    // there is none, which fails nothing
     void* scratch(size_t bytes)
     {
         void* d = nullptr;
         size_t cap = 0;
-        if (err_ || (err_ = mirrors().acquire(dev_, bytes, &d, &cap))) return nullptr;
+        if (err_ || mirrors().acquire(dev_, bytes, &d, &cap)) return nullptr;
         scratch_.emplace_back(cap, d);
         return d;
     }
@@ -125,7 +128,7 @@ public:
                     if (e.host && bytes > e.cap) {
                         mirrors().release(dev_, e.d, e.cap);
                         e.d = nullptr;
-                        if ((err_ = mirrors().acquire(dev_, bytes, &e.d, &e.cap))) return nullptr;
+                        if (!mirror(e)) return nullptr;
                     }
                 }
                 e.in |= in;
@@ -134,7 +137,7 @@ public:
             }
         Ent e{h, nullptr, bytes, 0, !on_device(h), in, out};
         if (e.host) {
-            if ((err_ = mirrors().acquire(dev_, bytes, &e.d, &e.cap))) return nullptr;
+            if (!mirror(e)) return nullptr;
         } else {
             e.d = const_cast<void*>(h);
         }
@@ -152,6 +155,12 @@ private:
         size_t bytes, cap;   // cap: the mirror's size (host arrays)
         bool host, in, out;
     };
+    bool mirror(Ent& e)
+    {
+        const int r = mirrors().acquire(dev_, e.bytes, &e.d, &e.cap);
+        if (r) err_ = cuda_fail((cudaError_t)r, "cudaMalloc(mirror)", __FILE__, __LINE__);
+        return r == 0;
+    }
     std::vector<Ent> ents_;
     std::vector<std::pair<size_t, void*>> scratch_;
     int dev_ = 0;   // the current device: the mirrors' and the kernels'
@@ -994,7 +1003,9 @@ static int do_expand(SE_FGG_work* w, const SE_state* st, const SE_FGG_params* p,
 }
 
 // The particles grouped by bin: `order`, and the bins' first places `off`
-// (bins.count + 2 entries, the stencils that leave the grid last).
+// (bins.count + 2 entries, the stencils that leave the grid last).  Both stay
+// null when there is no memory for them (24 bytes a particle): the callers then
+// keep the caller's order, which needs none.
 static int group_by_bin(Stager& s, const int* idx, const SE_FGG_params* p, const StencilBins& B, const int** off,
                         const int2** order)
 {
@@ -1003,7 +1014,7 @@ static int group_by_bin(Stager& s, const int* idx, const SE_FGG_params* p, const
     int4* slot = (int4*)s.scratch(sizeof(int4) * N);
     int2* ord = (int2*)s.scratch(sizeof(int2) * N);
     void* scan = s.scratch(std::max<size_t>(scan_scratch_bytes((long)nb), 16));
-    if (s.error()) return s.error();
+    if (!count || !slot || !ord || !scan) return s.error();
     SE_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * nb));
     k_bin_count<<<blocks(p->N, 256), 256>>>(idx, to_dev(p), B, count, slot);
     int launches = 0;
@@ -1054,11 +1065,10 @@ static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params
     const int* idx = (const int*)s.use(w->idx, 4 * (size_t)p->N, true, false);
     SE_TRY(s.copy_in());
     const StencilBins B(p);
-    if (windowed(p, B)) {
-        const int* off;
-        const int2* order;
-        SE_TRY(group_by_bin(s, idx, p, B, &off, &order));
-        const size_t smem = window_bytes(p->P);
+    const int* off = nullptr;
+    const int2* order = nullptr;
+    if (windowed(p, B)) SE_TRY(group_by_bin(s, idx, p, B, &off, &order));
+    if (order) {
         const auto fn = p->P == 16   ? k_grid_split_bins<16>
                         : p->P == 12 ? k_grid_split_bins<12>
                         : p->P == 8  ? k_grid_split_bins<8>
@@ -1134,7 +1144,7 @@ static int do_int_split(double* phi, const SE_FGG_work* w, const SE_FGG_params* 
     const int* idx = (const int*)s.use(w->idx, 4 * (size_t)p->N, true, false);
     SE_TRY(s.copy_in());
     const double h3 = p->h * p->h * p->h;
-    const int* off;
+    const int* off = nullptr;
     const int2* order = nullptr;
     if (grouped(p)) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
     const auto fn = p->P == 16   ? k_int_split<16>
@@ -1186,7 +1196,7 @@ static int do_int_split_force(double* force, const SE_state* st, const SE_FGG_wo
     const int* idx = (const int*)s.use(w->idx, 4 * (size_t)p->N, true, false);
     SE_TRY(s.copy_in());
     const double h3 = p->h * p->h * p->h;
-    const int* off;
+    const int* off = nullptr;
     const int2* order = nullptr;
     if (grouped(p)) SE_TRY(group_by_bin(s, idx, p, StencilBins(p), &off, &order));
     const auto fn = p->P == 16   ? k_int_split_force<16>
