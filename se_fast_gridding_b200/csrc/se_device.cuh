@@ -123,7 +123,7 @@ __device__ __forceinline__ int find_sys(const int* __restrict__ prefix, int nsys
 }
 
 // periodic index in [0, n) for any int i (SE_fgg.c:17-25 vmod)
-__device__ __forceinline__ int pmod(int i, int n)
+__host__ __device__ __forceinline__ int pmod(int i, int n)
 {
     const int r = i % n;
     return r < 0 ? r + n : r;

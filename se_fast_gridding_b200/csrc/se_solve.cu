@@ -560,16 +560,35 @@ static int path_of(const se_system* sys, const int* paths, int i)
     return paths ? paths[i] : default_path(sys[i].M, sys[i].P);
 }
 
-// Slab slots k_spread2 may need for a system, the parts after each tile's first:
-// at most the candidates of all its tiles over a part's, the candidates at most N
-// times the tiles that a bin's stencils (FB + P - 1 cells) reach -- 2 per axis on
-// whole tiles, else with a cut tile of one cell among them.
+// Tiles per axis that may have one bin's particles as candidates, at most.
+static int tiles_per_bin(int M, int P)
+{
+    const int nf = (M + FB - 1) / FB;
+    std::vector<int> tiles(nf, 0);
+    for (int o = 0; o < M; o += TX) {
+        const BinRanges r = bins_reaching(o, TX, M, P, nf);
+        for (int k = 0; k < range_count(r); k++) tiles[range_at(r, k)]++;
+    }
+    return *std::max_element(tiles.begin(), tiles.end());
+}
+
+// Slab slots k_spread2 may need for a system, the parts after each tile's first
+// (none where a tile's candidates, at most the N particles, are one part): at most
+// the candidates of all its tiles over a part's, and at most the parts of N
+// candidates in every tile.  A plan may later hold fewer particles, in smaller parts:
+// N / cap < most + 1, whatever N, and both bounds grow with N.
 static long long split_slots(const se_system& s, int path)
 {
-    const int cap = split_cap(path, s.M, s.P, s.N);
-    if (s.N <= cap || (!(path & PATH_TILE_SPREAD) && !spread2_general(path, s.M, s.P))) return 0;
-    const long long t = path & PATH_TILE_SPREAD ? 2 : (FB + s.P - 4) / TX + 3;
-    return t * t * t * s.N / cap;
+    if (!(path & PATH_TILE_SPREAD) && !spread2_general(path, s.M, s.P)) return 0;
+    if (s.N <= split_cap(path, s.M, s.P, s.N)) return 0;
+    const SplitRule r = split_rule(path, s.M, s.P, s.N);
+    const long long t = tiles_per_bin(s.M, s.P), nt = (s.M + TX - 1) / TX;
+    long long all = t * t * t * s.N / r.least, each = (s.N - 1) / r.least;
+    if (r.most) {
+        all = std::min(all, t * t * t * (r.most + 1));
+        each = std::min<long long>(each, r.most);
+    }
+    return std::min(all, nt * nt * nt * each);
 }
 
 static size_t batch_bytes(const se_system* sys, int nsys, int precision, int* nbins_out,

@@ -24,7 +24,7 @@ struct BinRanges {
     int a0, a1, b0, b1;   // [a0,a1] and [b0,b1]; b0 > b1 when absent
 };
 
-__device__ __forceinline__ BinRanges bins_reaching(int o, int T, int M, int P, int nf)
+__host__ __device__ __forceinline__ BinRanges bins_reaching(int o, int T, int M, int P, int nf)
 {
     BinRanges r;
     const int Ta = min(T, M - o);
@@ -46,12 +46,12 @@ __device__ __forceinline__ BinRanges bins_reaching(int o, int T, int M, int P, i
     return r;
 }
 
-__device__ __forceinline__ int range_count(const BinRanges& r)
+__host__ __device__ __forceinline__ int range_count(const BinRanges& r)
 {
     return (r.a1 - r.a0 + 1) + (r.b1 >= r.b0 ? r.b1 - r.b0 + 1 : 0);
 }
 
-__device__ __forceinline__ int range_at(const BinRanges& r, int k)
+__host__ __device__ __forceinline__ int range_at(const BinRanges& r, int k)
 {
     const int na = r.a1 - r.a0 + 1;
     return k < na ? r.a0 + k : r.b0 + (k - na);

@@ -68,18 +68,25 @@
 #define SE_S2_UNROLL 16
 #endif
 constexpr int S2_CAP = SE_S2_CAP;   // candidates per part of a warp's list
-// ... and of a system of N particles: off the whole tiles, where a particle is a
-// candidate of up to 4^3 or 5^3 tiles, at least N / 512, which bounds its slabs by 2
-// GB.  Where every block sees every particle (M <= P + 15: at most 27 tiles, which
-// leave the chip idle) parts of 512 from 1,025 particles on, or of N / 64 (slabs of
-// at most 256 MB): M = 32, P = 21, FP64 spread, 5,100 particles 0.467 -> 0.122 ms;
-// 1,024 (not split) 0.105, 1,088 0.098 (with parts of 1,024 0.128)
+// ... and of a system of N particles: at least `least`, and as many as make at most
+// `most` parts of all of them.  Off the whole tiles, where a particle is a candidate
+// of up to 4^3 tiles, 512 parts bound the slabs.  Where every block sees every
+// particle (M <= P + 15: at most 27 tiles, which leave the chip idle) parts of 512
+// from 1,025 particles on, or of N / 64: M = 32, P = 21, FP64 spread, 5,100 particles
+// 0.467 -> 0.122 ms; 1,024 (not split) 0.105, 1,088 0.098 (with parts of 1,024 0.128)
+struct SplitRule {
+    int least, most;   // most <= least
+};
+__host__ __device__ inline SplitRule split_rule(int path, int M, int P, int N)
+{
+    if (path & PATH_TILE_SPREAD) return {S2_CAP, 0};   // any number of parts
+    return M <= P + 15 && N > 1024 ? SplitRule{512, 64} : SplitRule{S2_CAP, 512};
+}
 __host__ __device__ inline int split_cap(int path, int M, int P, int N)
 {
-    if (path & PATH_TILE_SPREAD) return S2_CAP;
-    const bool few = M <= P + 15 && N > 1024;
-    const int least = few ? 512 : S2_CAP, even = N / (few ? 64 : 512);
-    return even < least ? least : even;
+    const SplitRule r = split_rule(path, M, P, N);
+    const int even = r.most ? N / r.most : 0;
+    return even < r.least ? r.least : even;
 }
 constexpr int S2_WARPS = 4;   // warp blocks per tile
 // warps per CTA: a tile's four warp blocks run as S2_WARPS / CW CTAs (the warps
