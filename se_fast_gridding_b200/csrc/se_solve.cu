@@ -440,7 +440,7 @@ struct se_batch_s {
         size_t smem = 0;
         bool mma = false;       // k_interp3
         bool tiled = false;     // from tile-aligned factor rows
-        int mode = SE_POTENTIAL;
+        int mode = SE_POTENTIAL;   // k_interp3: the systems' mode
         int units = 0;          // CTAs: the systems' bins / zb
         int* tab = nullptr;     // device: each unit's system, then its first bin
     };
@@ -851,8 +851,8 @@ static int interp2_table(se_batch_s* b, se_batch_s::I2Class& c, const std::vecto
 // The k_interp2 launches of a batch (se_batch_s::i2_cls).
 static int interp2_classes(se_batch_s* b, const se_system* systems, int nsys)
 {
-    // the systems of one launch: one stencil and mode each; those of
-    // k_interp2 in one launch when some system asks for runtime P
+    // the systems of one launch: one stencil each, and for k_interp3 one mode;
+    // those of k_interp2 in one launch when some system asks for runtime P
     struct Group {
         long long particles = 0, bins = 0;
         std::vector<int> members;
@@ -865,7 +865,7 @@ static int interp2_classes(se_batch_s* b, const se_system* systems, int nsys)
         const bool mma = interp3_better(S.path, b->precision, S.M, S.P, S.mode), tiled = S.path & PATH_PAIR_INTERP;
         if (!mma && !tiled) continue;
         const bool any_p = b->runtime_p && !mma;
-        Group& g = groups[{mma, tiled, any_p ? 0 : S.P, any_p ? 0 : S.mode}];
+        Group& g = groups[{mma, tiled, any_p ? 0 : S.P, mma ? S.mode : SE_POTENTIAL}];
         g.particles += S.N;
         g.bins += (long long)S.nf[0] * S.nf[1] * S.nf[2];
         g.members.push_back(i);

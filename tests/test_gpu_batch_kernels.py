@@ -45,3 +45,18 @@ def test_crowded_bins_of_another_kernel(env, systems):
         se.close()
         np.testing.assert_array_equal(out, one)
 
+
+def test_mixed_modes_take_no_more_launches(env):
+    """k_interp2 serves potentials and forces of one stencil in one launch."""
+    import oracle as O
+    torch, S = env
+    count = {}
+    for modes in (("force", "force"), ("potential", "force")):
+        sy = [S.System(500, 64, P, 1.0, 8.0, None, mode) for P in (8, 12, 16) for mode in modes]
+        b = S.BatchSolver(sy, "fp32")
+        x, q = b.pack(*zip(*[O.synthetic_system(s.N, 1.0, seed=k) for k, s in enumerate(sy)]))
+        b.solve(x, q)
+        torch.cuda.synchronize()
+        count[modes] = b.launches
+        b.close()
+    assert len(set(count.values())) == 1, count
