@@ -10,7 +10,8 @@
 //               order for every target;
 //   cell list   0 < rc <= L/2 with at least 3 cells of edge >= rc per axis:
 //               particles sorted by cell (the library's stable sort), one
-//               warp per target (in cell order) over the 27 neighbour cells.
+//               warp per target (in cell order), or one thread for many
+//               targets of few neighbours, over the 27 neighbour cells.
 //               Each particle keeps its position wrapped into the box and the
 //               number of boxes it was moved by, so the image of a pair is
 //               recovered exactly and the reference's limit |p| <= layers on
@@ -112,13 +113,20 @@ __global__ void k_real_keys(RsParams S, int nc, const double* __restrict__ x,
     key[n] = (c[0] * nc + c[1]) * nc + c[2];
 }
 
+// The groups of 32 targets left to k_real_cells_crowded, and its next target.
+struct RsCrowded {
+    int groups, next;
+};
+
 // Sorted records: wrapped position and charge, and the box shifts k_a =
 // floor(x_a / L) (each within +-511).
 __global__ void k_real_gather(RsParams S, const int* __restrict__ perm,
                               const double* __restrict__ x, const double* __restrict__ q,
-                              double4* __restrict__ rec, int* __restrict__ kbox)
+                              double4* __restrict__ rec, int* __restrict__ kbox,
+                              RsCrowded* __restrict__ crowded)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s == 0 && crowded) *crowded = {};
     if (s >= S.N) return;
     const int n = perm[s];
     double w[3];
@@ -135,70 +143,84 @@ __global__ void k_real_gather(RsParams S, const int* __restrict__ perm,
 
 __device__ __forceinline__ int kbox_of(int pk, int a) { return ((pk >> (10 * a)) & 1023) - 512; }
 
-// One warp per target (in cell order).  The lanes test 32 candidates of the
-// neighbour cells at a time -- a row of up to three z cells is one run of the
-// sorted particles -- and queue the pairs inside the cutoff; 32 queued pairs
-// are then evaluated together, one per lane.  About one candidate in eight is
-// a pair, and a pair costs some ten times a test (erfc, exp, two divisions):
-// with a target per thread most lanes of a warp sat out every evaluation
+// The candidates of a target in cell c are 18 runs of the sorted particles: run u
+// holds the z cells c[2] - 1 to c[2] + 1 of neighbour row u / 2 (u even), or the one of
+// them past the box's end (u odd, else empty).  shift: the run's box shifts + 1, 2
+// bits an axis.
+__device__ __forceinline__ void neighbour_run(int u, const int c[3], int nc, const int* __restrict__ cell_off,
+                                              int& beg, int& end, int& shift)
+{
+    const int cx = c[0] + u / 6 - 1, cy = c[1] + u / 2 % 3 - 1;
+    const int sh0 = cx < 0 ? -1 : (cx >= nc ? 1 : 0);
+    const int sh1 = cy < 0 ? -1 : (cy >= nc ? 1 : 0);
+    const int row = ((cx - sh0 * nc) * nc + cy - sh1 * nc) * nc;
+    int z0 = max(c[2] - 1, 0), z1 = min(c[2] + 1, nc - 1);
+    int sh2 = 0;
+    if (u & 1) {
+        sh2 = c[2] == 0 ? -1 : (c[2] == nc - 1 ? 1 : 0);
+        z0 = c[2] == 0 ? nc - 1 : 0;
+        z1 = sh2 ? z0 : z0 - 1;
+    }
+    beg = cell_off[row + z0];
+    end = cell_off[row + z1 + 1];
+    shift = (sh0 + 1) | (sh1 + 1) << 2 | (sh2 + 1) << 4;
+}
+
+// Separation of the target at xm from particle o of a run, and its square.
+__device__ __forceinline__ double separation(const RsParams& S, const double xm[3], const double4& o, int shift,
+                                             double (&d)[3])
+{
+    d[0] = xm[0] - (o.x + ((shift & 3) - 1) * S.L);
+    d[1] = xm[1] - (o.y + ((shift >> 2 & 3) - 1) * S.L);
+    d[2] = xm[2] - (o.z + ((shift >> 4 & 3) - 1) * S.L);
+    return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+}
+
+// The term of a pair inside the cutoff, e: the particle and its run's shifts.
+template <bool FORCE>
+__device__ __forceinline__ void queued_pair(const RsParams& S, const double xm[3], int km,
+                                            const double4* __restrict__ rec, const int* __restrict__ kbox, int2 e,
+                                            double& acc, double (&f)[3])
+{
+    const double4 o = rec[e.x];
+    const int kt = kbox[e.x];
+    double d[3];
+    const double rr = separation(S, xm, o, e.y, d);
+    bool in = true;   // the image index of the pair in raw coordinates
+    for (int a = 0; a < 3; a++) {
+        const int p = kbox_of(kt, a) - kbox_of(km, a) - ((e.y >> 2 * a & 3) - 1);
+        in = in && p >= -S.layers && p <= S.layers;
+    }
+    if (in) pair_term<FORCE>(S, o.w, d, rr, acc, f);
+}
+
+// One warp per target s (in cell order).  The lanes test 32 candidates of the
+// neighbour cells at a time and queue the pairs inside the cutoff; 32 queued pairs
+// are then evaluated together, one per lane.  About one candidate in eight is a pair,
+// and a pair costs some ten times a test (erfc, exp, two divisions): with a target per
+// thread, its pairs evaluated as they are found, most lanes sat out every evaluation
 // (50,000 particles, about 100 neighbours each, force: 548 -> 205 us; the FP64
 // pipe 35% and the issue slots 65% busy; with the separations queued instead
 // of the particles, 246 us).
 // A lane sums its pairs in queue order and the lanes' sums are added in a
 // fixed order, so results are deterministic.
 template <bool FORCE>
-__global__ void __launch_bounds__(RS_THREADS) k_real_cells(
-    RsParams S, int nc, const double4* __restrict__ rec, const int* __restrict__ kbox,
-    const int* __restrict__ perm, const int* __restrict__ cell_off, double* __restrict__ phi,
-    double* __restrict__ force)
+__device__ __forceinline__ void target_by_warp(const RsParams& S, int nc, const double4* __restrict__ rec,
+                                               const int* __restrict__ kbox, const int* __restrict__ perm,
+                                               const int* __restrict__ cell_off, double* __restrict__ phi,
+                                               double* __restrict__ force, int s, int2* que)
 {
-    __shared__ int2 queue[RS_THREADS / 32][64];   // particle, box shifts + 1 (2 bits an axis)
-    const int s = blockIdx.x * (RS_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (s >= S.N) return;
-    int2* que = queue[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
     const double4 me = rec[s];
     const int km = kbox[s];
     const double xm[3] = {me.x, me.y, me.z};
     int c[3];
     for (int a = 0; a < 3; a++) c[a] = min((int)(xm[a] * nc / S.L), nc - 1);
-    // lane l < 18: run l, the z cells below or above the box's end (l odd) or
-    // the others of neighbour row l / 2, and its box shifts
+    // lane l < 18: run l and its box shifts
     int beg = 0, end = 0, shift = 0;
-    if (lane < 18) {
-        const int cx = c[0] + lane / 6 - 1, cy = c[1] + lane / 2 % 3 - 1;
-        const int sh0 = cx < 0 ? -1 : (cx >= nc ? 1 : 0);
-        const int sh1 = cy < 0 ? -1 : (cy >= nc ? 1 : 0);
-        const int row = ((cx - sh0 * nc) * nc + cy - sh1 * nc) * nc;
-        int z0 = max(c[2] - 1, 0), z1 = min(c[2] + 1, nc - 1);
-        int sh2 = 0;
-        if (lane & 1) {
-            sh2 = c[2] == 0 ? -1 : (c[2] == nc - 1 ? 1 : 0);
-            z0 = c[2] == 0 ? nc - 1 : 0;
-            z1 = sh2 ? z0 : z0 - 1;
-        }
-        beg = cell_off[row + z0];
-        end = cell_off[row + z1 + 1];
-        shift = (sh0 + 1) | (sh1 + 1) << 2 | (sh2 + 1) << 4;
-    }
+    if (lane < 18) neighbour_run(lane, c, nc, cell_off, beg, end, shift);
     double acc = 0, f[3] = {0, 0, 0};
-    auto separation = [&](const double4& o, int sh, double (&d)[3]) {
-        d[0] = xm[0] - (o.x + ((sh & 3) - 1) * S.L);
-        d[1] = xm[1] - (o.y + ((sh >> 2 & 3) - 1) * S.L);
-        d[2] = xm[2] - (o.z + ((sh >> 4 & 3) - 1) * S.L);
-        return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    };
-    auto pair = [&](int2 e) {
-        const double4 o = rec[e.x];
-        const int kt = kbox[e.x];
-        double d[3];
-        const double rr = separation(o, e.y, d);
-        bool in = true;   // the image index of the pair in raw coordinates
-        for (int a = 0; a < 3; a++) {
-            const int p = kbox_of(kt, a) - kbox_of(km, a) - ((e.y >> 2 * a & 3) - 1);
-            in = in && p >= -S.layers && p <= S.layers;
-        }
-        if (in) pair_term<FORCE>(S, o.w, d, rr, acc, f);
-    };
+    auto pair = [&](int2 e) { queued_pair<FORCE>(S, xm, km, rec, kbox, e, acc, f); };
     int queued = 0;
     for (int run = 0; run < 18; run++) {
         const int b = __shfl_sync(0xffffffffu, beg, run), e = __shfl_sync(0xffffffffu, end, run);
@@ -208,7 +230,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_real_cells(
             const int t = t0 + lane;
             double d[3];
             // (a particle is in one cell, so t = s is the pair with itself)
-            const bool in = t < e && t != s && !(separation(rec[min(t, e - 1)], sh, d) > S.rc2);
+            const bool in = t < e && t != s && !(separation(S, xm, rec[min(t, e - 1)], sh, d) > S.rc2);
             const unsigned hit = __ballot_sync(0xffffffffu, in);
             if (in) que[queued + __popc(hit & ((1u << lane) - 1u))] = make_int2(t, sh);
             queued += __popc(hit);
@@ -240,6 +262,109 @@ __global__ void __launch_bounds__(RS_THREADS) k_real_cells(
     }
 }
 
+template <bool FORCE>
+__global__ void __launch_bounds__(RS_THREADS) k_real_cells(
+    RsParams S, int nc, const double4* __restrict__ rec, const int* __restrict__ kbox,
+    const int* __restrict__ perm, const int* __restrict__ cell_off, double* __restrict__ phi,
+    double* __restrict__ force)
+{
+    __shared__ int2 queue[RS_THREADS / 32][64];   // particle, box shifts + 1 (2 bits an axis)
+    const int warp = threadIdx.x >> 5, s = blockIdx.x * (RS_THREADS / 32) + warp;
+    if (s < S.N) target_by_warp<FORCE>(S, nc, rec, kbox, perm, cell_off, phi, force, s, queue[warp]);
+}
+
+// One thread per target, for many targets of few candidates each.  A lane queues its
+// own pairs inside the cutoff and the lanes of a warp evaluate theirs together,
+// when some lane's queue is full (straight from the test, a warp pays for a pair
+// whenever one lane has one).  A warp with a target of more than RS_CROWDED candidates
+// leaves its targets to k_real_cells_crowded.
+constexpr int RS_QUEUE = 16;
+constexpr int RS_CROWDED = 224;
+constexpr int RS_CROWDED_CTAS = 148 * 12;   // (as many as are resident, and more)
+
+template <bool FORCE>
+__global__ void __launch_bounds__(RS_THREADS) k_real_cells_sparse(
+    RsParams S, int nc, const double4* __restrict__ rec, const int* __restrict__ kbox,
+    const int* __restrict__ perm, const int* __restrict__ cell_off, double* __restrict__ phi,
+    double* __restrict__ force, RsCrowded* __restrict__ crowded, int* __restrict__ group)
+{
+    __shared__ int2 queue[RS_THREADS / 32][RS_QUEUE][32];
+    int2(*que)[32] = queue[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int s = blockIdx.x * RS_THREADS + threadIdx.x;
+    const bool on = s < S.N;   // (the other lanes of the last warp have no candidates)
+    const double4 me = rec[on ? s : 0];
+    const int km = kbox[on ? s : 0];
+    const double xm[3] = {me.x, me.y, me.z};
+    int c[3];
+    for (int a = 0; a < 3; a++) c[a] = min((int)(xm[a] * nc / S.L), nc - 1);
+    int candidates = 0;
+    if (on)
+        for (int run = 0; run < 18; run++) {
+            int beg, end, shift;
+            neighbour_run(run, c, nc, cell_off, beg, end, shift);
+            candidates += end - beg;
+        }
+    if (__any_sync(0xffffffffu, candidates > RS_CROWDED)) {
+        if (lane == 0) group[atomicAdd(&crowded->groups, 1)] = s >> 5;
+        return;
+    }
+    double acc = 0, f[3] = {0, 0, 0};
+    int queued = 0;
+    auto flush = [&] {
+        for (int i = 0; __any_sync(0xffffffffu, i < queued); i++)
+            if (i < queued) queued_pair<FORCE>(S, xm, km, rec, kbox, que[i][lane], acc, f);
+        queued = 0;
+    };
+    for (int run = 0; run < 18; run++) {
+        int beg = 0, end = 0, shift = 0;
+        if (on) neighbour_run(run, c, nc, cell_off, beg, end, shift);
+        for (int t0 = beg; __any_sync(0xffffffffu, t0 < end); t0 += 2) {
+            double4 o[2];   // (two loads in flight)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                if (t0 + j < end) o[j] = rec[t0 + j];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int t = t0 + j;
+                double d[3];
+                if (t < end && t != s && !(separation(S, xm, o[j], shift, d) > S.rc2))
+                    que[queued++][lane] = make_int2(t, shift);
+            }
+            if (__any_sync(0xffffffffu, queued > RS_QUEUE - 2)) flush();
+        }
+    }
+    flush();
+    if (!on) return;
+    const int m = perm[s];
+    if (phi) phi[m] += acc;
+    if (FORCE) {
+        force[m] += me.w * f[0];
+        force[m + S.N] += me.w * f[1];
+        force[m + 2 * S.N] += me.w * f[2];
+    }
+}
+
+// The targets of the listed groups, a warp each, as the warps get free.
+template <bool FORCE>
+__global__ void __launch_bounds__(RS_THREADS) k_real_cells_crowded(
+    RsParams S, int nc, const double4* __restrict__ rec, const int* __restrict__ kbox,
+    const int* __restrict__ perm, const int* __restrict__ cell_off, double* __restrict__ phi,
+    double* __restrict__ force, RsCrowded* __restrict__ crowded, const int* __restrict__ group)
+{
+    __shared__ int2 queue[RS_THREADS / 32][64];
+    const int groups = crowded->groups;
+    for (;;) {
+        int t = 0;
+        if ((threadIdx.x & 31) == 0) t = atomicAdd(&crowded->next, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >> 5 >= groups) return;
+        const int s = 32 * group[t >> 5] + (t & 31);
+        if (s < S.N) target_by_warp<FORCE>(S, nc, rec, kbox, perm, cell_off, phi, force, s, queue[threadIdx.x >> 5]);
+        __syncwarp();   // its queue is used again
+    }
+}
+
 __global__ void k_self(const double* __restrict__ q, int N, double c, double* __restrict__ phi)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,6 +377,20 @@ int cells_per_axis(double L, double rc)
     if (!(rc > 0) || 2 * rc > L) return 0;
     const double nc = floor(L / rc);
     return (nc >= 3 && nc <= 256) ? (int)nc : 0;
+}
+
+// Whether the targets go a thread each (k_real_cells_sparse) where they are not
+// crowded: from 2^18 particles on and up to 160 candidates on average.  A warp and a
+// thread per target, force, us: 2M uniform particles with 1, 6, 15 and 25
+// neighbours (6 to 160 candidates) 3331, 4021, 4157, 4133 and 735, 1006, 1709, 2490;
+// 300,000 with 1, 15 and 50 600, 716, 880 and 245, 438, 902; 30,000 with 1 and 10
+// 150, 142 and 127, 141, 3,000 with 1 86 and 98.  1M clustered (16 Gaussians of sigma
+// 0.03; 5 neighbours on average, most targets left to k_real_cells_crowded) 6649
+// and 6609, potentials alone 5297 and 5932; with 140,000 of them the warps left to the
+// thread kernel are its whole time: 385 and 570.
+static bool sparse_targets(int N, int ncell)
+{
+    return N >= 1 << 18 && 27.0 * N <= 160.0 * ncell;
 }
 
 // Scratch of a call, ordered on its stream: from a pool of this library's own
@@ -339,10 +478,20 @@ int real_space(const double* x, const double* q, int N, double L, double xi, int
     if (e == cudaSuccess) {
         r = stable_sort(key, nullptr, N, ncell, perm, nullptr, off, scratch, sb, st, nullptr);
         if (r == SE_OK) {
-            k_real_gather<<<ceil_div(N, 256), 256, 0, st>>>(S, perm, x, q, rec, kbox);
-            const unsigned nw = ceil_div(N, RS_THREADS / 32);
-            if (force) k_real_cells<true><<<nw, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, phi, force);
-            else k_real_cells<false><<<nw, RS_THREADS, 0, st>>>(S, nc, rec, kbox, perm, off, phi, nullptr);
+            // (the keys are of no more use: the crowded groups' list in their place)
+            const bool sparse = sparse_targets(N, ncell);
+            RsCrowded* crowded = sparse ? reinterpret_cast<RsCrowded*>(key) : nullptr;
+            int* group = key + sizeof(RsCrowded) / sizeof(int);
+            k_real_gather<<<ceil_div(N, 256), 256, 0, st>>>(S, perm, x, q, rec, kbox, crowded);
+            if (sparse) {
+                (force ? k_real_cells_sparse<true> : k_real_cells_sparse<false>)<<<nb, RS_THREADS, 0, st>>>(
+                    S, nc, rec, kbox, perm, off, phi, force, crowded, group);
+                (force ? k_real_cells_crowded<true> : k_real_cells_crowded<false>)<<<RS_CROWDED_CTAS, RS_THREADS, 0, st>>>(
+                    S, nc, rec, kbox, perm, off, phi, force, crowded, group);
+            } else {
+                (force ? k_real_cells<true> : k_real_cells<false>)<<<ceil_div(N, RS_THREADS / 32), RS_THREADS, 0, st>>>(
+                    S, nc, rec, kbox, perm, off, phi, force);
+            }
             e = cudaGetLastError();
         }
     }
