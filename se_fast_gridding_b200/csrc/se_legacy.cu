@@ -345,47 +345,57 @@ __device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int 
     return corner;
 }
 
-// SE_fgg.c:920-963 (q = 1).  A warp expands 32 particles, one per lane; the
-// rows go through shared memory so that they are stored P consecutive values
-// at a time (stored by their own lanes, P values apart: 30,000 particles, P =
-// 16, force, B200: 26 -> 15 us).
-constexpr int EXPAND_WARPS = 4;
+// SE_fgg.c:920-963 (q = 1).  A warp expands 32 particles, one per lane, the three
+// axes' powers side by side; the rows, which lie one after the other in memory,
+// go through shared memory and are stored 32 consecutive values at a time (by their own
+// lanes, P values apart, and row by row: call on 400,000 particles, P = 2, force, 55 and
+// 100 us, now 57; 1,000, P = 4 39, 47 and 41; 30,600, P = 16, force 61, 49 and 49).
+static size_t expand_bytes(int P) { return sizeof(double) * 3 * 32 * (size_t)(P | 1); }
 
-__global__ void __launch_bounds__(EXPAND_WARPS * 32) k_expand_all(
+__global__ void __launch_bounds__(32) k_expand_all(
     ParamsDev p, const double* __restrict__ x, int periodicity, double* zx, double* zy, double* zz,
     double* zfx, double* zfy, double* zfz, int* idx)
 {
-    __shared__ double row[EXPAND_WARPS][32][SE_P_MAX + 1];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (blockIdx.x * EXPAND_WARPS + w) * 32, n = min(n0 + lane, p.N - 1);
-    const int cnt = min(32, p.N - n0);
-    if (cnt <= 0) return;
+    extern __shared__ double row[];   // [axis][particle][pitch]
+    __shared__ double ts[3][32];
+    const int P = p.P, pitch = P | 1, lane = threadIdx.x;
+    const int n0 = blockIdx.x * 32, n = min(n0 + lane, p.N - 1), cnt = min(32, p.N - n0);
     const double xn[3] = {x[n], x[n + p.N], x[n + 2 * p.N]};
-    double t0[3];
-    double* zs[3] = {zx, zy, zz};
-    double* zf[3] = {zfx, zfy, zfz};
+    double t0[3], v[3], base[3];
     const int corner = expand_corner(xn, p, periodicity, t0);
     if (lane < cnt) idx[n] = corner;
     const double z3 = exp(-p.c * (t0[0] * t0[0] + t0[1] * t0[1] + t0[2] * t0[2]));
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        const double base = exp(2 * p.c * p.h * t0[d]);
-        double v = pow(base, (double)p.lo);
-        row[w][lane][0] = d == 0 ? v * z3 : v;
-        for (int i = 1; i < p.P; i++) {
-            v *= base;
-            row[w][lane][i] = d == 0 ? v * z3 : v;
+        ts[d][lane] = t0[d];
+        base[d] = exp(2 * p.c * p.h * t0[d]);
+        v[d] = pow(base[d], (double)p.lo);
+    }
+    for (int i = 0; i < P; i++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            row[(d * 32 + lane) * pitch + i] = d == 0 ? v[d] * z3 : v[d];
+            v[d] *= base[d];
         }
-        __syncwarp();
-        for (int r = 0; r < cnt; r++) {
-            const double t = __shfl_sync(0xffffffffu, t0[d], r);
-            if (lane < p.P) {
-                const long long o = (long long)(n0 + r) * p.P + lane;
-                zs[d][o] = row[w][r][lane];
-                if (zf[d]) zf[d][o] = -p.c * (t - (p.lo + lane) * p.h);
+    __syncwarp();
+    double* zs[3] = {zx, zy, zz};
+    double* zf[3] = {zfx, zfy, zfz};
+    const int dr = 32 / P, dk = 32 % P;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        double* z = zs[d] + (long long)n0 * P;
+        double* f = zf[d] ? zf[d] + (long long)n0 * P : nullptr;
+        int r = lane / P, k = lane % P;
+        for (int e = lane; e < cnt * P; e += 32) {
+            z[e] = row[(d * 32 + r) * pitch + k];
+            if (f) f[e] = -p.c * (ts[d][r] - (p.lo + k) * p.h);
+            r += dr;
+            k += dk;
+            if (k >= P) {
+                k -= P;
+                r++;
             }
         }
-        __syncwarp();
     }
 }
 
@@ -997,7 +1007,7 @@ static int do_expand(SE_FGG_work* w, const SE_state* st, const SE_FGG_params* p,
     double* fz = force ? (double*)s.use(w->zfz, NP * 8, false, true) : nullptr;
     int* idx = (int*)s.use(w->idx, 4 * (size_t)p->N, false, true);
     SE_TRY(s.copy_in());
-    k_expand_all<<<blocks(p->N, EXPAND_WARPS * 32), EXPAND_WARPS * 32>>>(
+    k_expand_all<<<blocks(p->N, 32), 32, expand_bytes(p->P)>>>(
         to_dev(p), x, periodicity, zx, zy, zz, fx, fy, fz, idx);
     return s.finish();
 }
