@@ -432,15 +432,56 @@ struct StencilLane {
     }
 };
 
+// The walk of small stencils, whose rows leave lanes of a warp idle: the cells in order,
+// 32 at a time, their indices carried along.
+constexpr int SMALL_STENCIL = -1;   // PT of this walk
+
+struct SmallStencilWalk {
+    int P, i, j, k, di, dj, dk;
+    __device__ __forceinline__ SmallStencilWalk(int p) : P(p)
+    {
+        const int lane = threadIdx.x & 31, inv = (65536 + P - 1) / P;
+        auto over = [&](int v) { return v * inv >> 16; };   // v / P, v <= 32
+        const int lp = over(lane), cp = over(32);
+        i = over(lp);
+        j = lp - i * P;
+        k = lane - lp * P;
+        di = over(cp);   // 32 cells on
+        dj = cp - di * P;
+        dk = 32 - cp * P;
+    }
+    __device__ __forceinline__ void step()
+    {
+        k += dk;
+        const int cj = k >= P;
+        k -= cj ? P : 0;
+        j += dj + cj;
+        const int ci = j >= P;
+        j -= ci ? P : 0;
+        i += di + ci;
+    }
+};
+
 // H[cell] += zs[cell] zz[k] (q zx[i] zy[j]), or the product order of
-// SE_fgg.c:4964-5009 (force_order) instead of that of :3983-4028.
+// SE_fgg.c:4964-5009 (force_order) instead of that of :3983-4028, on the x planes
+// i0, i0 + istep, ... (with SMALL_STENCIL on all of them)
 template <int PT>
 __device__ __forceinline__ void scatter_stencil(double* H, long long base, int p, int n1, int n2,
                                                 const double* __restrict__ zs, const double* zx,
                                                 const double* zy, const double* zz, double q,
-                                                int force_order)
+                                                int force_order, int i0, int istep)
 {
-    const StencilLane<PT> L(p);
+    if constexpr (PT == SMALL_STENCIL) {
+        SmallStencilWalk W(p);
+        for (int s = threadIdx.x & 31; s < p * p * p; s += 32, W.step()) {
+            const double x = force_order ? zx[W.i] : q * zx[W.i];
+            double v = zs[s] * zz[W.k] * (x * zy[W.j]);
+            if (force_order) v *= q;
+            atomicAdd(H + base + ((long long)W.i * n1 + W.j) * n2 + W.k, v);
+        }
+        return;
+    }
+    const StencilLane<PT == SMALL_STENCIL ? 0 : PT> L(p);
     const int P = L.P;
     if (!L.on) return;
     const double zk = zz[L.k];
@@ -448,9 +489,9 @@ __device__ __forceinline__ void scatter_stencil(double* H, long long base, int p
         double y[STENCIL_ROWS];
 #pragma unroll
         for (int m = 0; m < STENCIL_ROWS; m++) y[m] = L.row(jc, m) ? zy[jc + m * L.R] : 0.0;
-        const double* z = zs + jc * P + L.k;
-        double* h = H + base + (long long)jc * n2 + L.k;
-        for (int i = 0; i < P; i++, z += P * P, h += (long long)n1 * n2) {
+        const double* z = zs + (i0 * P + jc) * P + L.k;
+        double* h = H + base + ((long long)i0 * n1 + jc) * n2 + L.k;
+        for (int i = i0; i < P; i += istep, z += istep * P * P, h += (long long)istep * n1 * n2) {
             const double x = force_order ? zx[i] : q * zx[i];
             double v[STENCIL_ROWS];
 #pragma unroll
@@ -473,7 +514,22 @@ __device__ __forceinline__ void gather_stencil(const double* __restrict__ H, lon
                                                const double* zy, const double* zz, const double* zfx,
                                                const double* zfy, const double* zfz, double (&a)[4])
 {
-    const StencilLane<PT> L(p);
+    if constexpr (PT == SMALL_STENCIL) {
+        SmallStencilWalk W(p);
+        a[0] = a[1] = a[2] = a[3] = 0.0;
+#pragma unroll (FORCE ? 1 : 2)
+        for (int s = threadIdx.x & 31; s < p * p * p; s += 32, W.step()) {
+            const double v = H[base + ((long long)W.i * n1 + W.j) * n2 + W.k] * zs[s] * zz[W.k] * (zx[W.i] * zy[W.j]);
+            a[0] += v;
+            if (FORCE) {
+                a[1] = fma(v, zfx[W.i], a[1]);
+                a[2] = fma(v, zfy[W.j], a[2]);
+                a[3] = fma(v, zfz[W.k], a[3]);
+            }
+        }
+        return;
+    }
+    const StencilLane<PT == SMALL_STENCIL ? 0 : PT> L(p);
     const int P = L.P;
     a[0] = a[1] = a[2] = a[3] = 0.0;
     if (!L.on) return;
@@ -519,15 +575,17 @@ __device__ __forceinline__ void gather_stencil(const double* __restrict__ H, lon
     }
 }
 
-// Scatter of one particle's P^3 stencil per warp.
+// Scatter of one particle's P^3 stencil per warp (SPREAD: per CTA, its warps taking
+// the x planes in turn).
 constexpr int SCATTER_WARPS = 8;
 
+template <bool SPREAD, int PT>
 __global__ void __launch_bounds__(SCATTER_WARPS * 32) k_grid_split(
     double* H, const double* __restrict__ q, const double* __restrict__ zs, const double* __restrict__ zx,
     const double* __restrict__ zy, const double* __restrict__ zz, const int* __restrict__ idx, ParamsDev p,
     int force_order)
 {
-    const int n = blockIdx.x * SCATTER_WARPS + (threadIdx.x >> 5);
+    const int w = threadIdx.x >> 5, n = SPREAD ? blockIdx.x : blockIdx.x * SCATTER_WARPS + w;
     if (n >= p.N) return;
     const long long o = (long long)n * p.P;
     const long long base = idx[n];
@@ -535,30 +593,35 @@ __global__ void __launch_bounds__(SCATTER_WARPS * 32) k_grid_split(
         if ((threadIdx.x & 31) == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    scatter_stencil<0>(H, base, p.P, p.npdims[1], p.npdims[2], zs, zx + o, zy + o, zz + o, q[n], force_order);
+    scatter_stencil<PT>(H, base, p.P, p.npdims[1], p.npdims[2], zs, zx + o, zy + o, zz + o, q[n], force_order,
+                        SPREAD ? w : 0, SPREAD ? SCATTER_WARPS : 1);
 }
 
 // SE_fgg.c:3866-3914: expansion with the charge, then the same scatter
+template <bool SPREAD>
 __global__ void __launch_bounds__(SCATTER_WARPS * 32) k_grid_vanilla(
     double* H, const double* __restrict__ x, const double* __restrict__ q, const double* __restrict__ zs,
     ParamsDev p, int periodicity)
 {
-    __shared__ double zsm[SCATTER_WARPS][3][SE_P_MAX];
-    __shared__ int c0s[SCATTER_WARPS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = blockIdx.x * SCATTER_WARPS + w;
-    if (n >= p.N) return;
-    double(&z)[3][SE_P_MAX] = zsm[w];
-    if (lane == 0) {
+    constexpr int PARTICLES = SPREAD ? 1 : SCATTER_WARPS;
+    __shared__ double zsm[PARTICLES][3][SE_P_MAX];
+    __shared__ int c0s[PARTICLES];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, own = SPREAD ? 0 : w;
+    const int n = blockIdx.x * PARTICLES + own;
+    if (n >= p.N) return;   // (all of a SPREAD CTA or none)
+    double(&z)[3][SE_P_MAX] = zsm[own];
+    if (lane == 0 && w == own) {
         const double xn[3] = {x[n], x[n + p.N], x[n + 2 * p.N]};
-        c0s[w] = expand_one(xn, q[n], p, periodicity, z[0], z[1], z[2], nullptr, nullptr, nullptr);
+        c0s[own] = expand_one(xn, q[n], p, periodicity, z[0], z[1], z[2], nullptr, nullptr, nullptr);
     }
-    __syncwarp();
-    if (!stencil_in_bounds(c0s[w], p)) {
+    if (SPREAD) __syncthreads();
+    else __syncwarp();
+    if (!stencil_in_bounds(c0s[own], p)) {
         if (lane == 0) atomicOr(&g_legacy_err, 1);
         return;
     }
-    scatter_stencil<0>(H, c0s[w], p.P, p.npdims[1], p.npdims[2], zs, z[0], z[1], z[2], 1.0, 0);
+    scatter_stencil<0>(H, c0s[own], p.P, p.npdims[1], p.npdims[2], zs, z[0], z[1], z[2], 1.0, 0, SPREAD ? w : 0,
+                       SPREAD ? SCATTER_WARPS : 1);
 }
 
 // ---- particles grouped by the 8^3 bin of their padded corner
@@ -1039,10 +1102,12 @@ static int group_by_bin(Stager& s, const int* idx, const SE_FGG_params* p, const
 // Whether the particles are grouped for a gather.  Grouping takes three
 // launches, 13 us; the gather of 30,000 particles at P = 16 (1.2e8 stencil cells)
 // took 370 us in the caller's order and one load at a time, 231 us grouped and
-// eight loads ahead, 165 us with P compiled in.
+// eight loads ahead, 165 us with P compiled in.  Stencils of P < 8 gain nothing by it
+// (500,000 particles, P = 4: 201 us in the caller's order, 246 to 348 grouped; P = 6
+// 344 and 384 to 468).
 static bool grouped(const SE_FGG_params* p)
 {
-    return (double)p->N * p->P * p->P * p->P >= 1.6e7;
+    return p->P >= 8 && (double)p->N * p->P * p->P * p->P >= 1.6e7;
 }
 
 // Whether a scatter goes through shared-memory windows: where they have far
@@ -1057,6 +1122,18 @@ static bool windowed(const SE_FGG_params* p, const StencilBins& B)
     return grouped(p) && p->P <= WINDOW_MAX_P &&
            W * W * W * B.count * 2.0 < (double)p->N * P * P * P;
 }
+
+// Whether a CTA, not a warp, scatters each particle: where a warp each would leave
+// the chip idle and a particle's P^3 cells take long one warp after another.
+// Scatter call, us, a warp and a CTA each: P = 32 300: 114, 59, 10,000: 635, 595; P =
+// 21 100: 69, 44, 6,000: 151, 143; P = 16 300: 49, 40, 4,000: 82, 71; P = 12 300: 44,
+// 39, 2,500: 50, 50; P = 8 300: 42, 40, 2,500: 42, 48; P = 4 1,500: 41, 44.
+static bool scatter_spread(const SE_FGG_params* p) { return p->N <= 16 * p->P * p->P; }
+
+// The same with the expansion in the scatter, which every CTA waits for: P = 32 1,500:
+// 162, 133, 4,000: 382, 275; P = 21 1,000: 75, 63, 2,500: 94, 92; P = 16 700: 51, 50,
+// 1,500: 56, 57; P = 12 700: 46, 47, 1,500: 50, 53; P = 8 300: 43, 41, 1,000: 44, 46.
+static bool scatter_vanilla_spread(const SE_FGG_params* p) { return p->N <= 64 * p->P; }
 
 static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params* p,
                          int force_order)
@@ -1089,7 +1166,11 @@ static int do_grid_split(SE_FGG_work* w, const SE_state* st, const SE_FGG_params
             H, q, zs, zx, zy, zz, to_dev(p), B, off, order, force_order);
         return s.finish();
     }
-    k_grid_split<<<blocks(p->N, SCATTER_WARPS), SCATTER_WARPS * 32>>>(
+    const bool spread = scatter_spread(p);
+    const auto fn = spread     ? k_grid_split<true, 0>
+                    : p->P < 8 ? k_grid_split<false, SMALL_STENCIL>
+                               : k_grid_split<false, 0>;
+    fn<<<spread ? p->N : blocks(p->N, SCATTER_WARPS), SCATTER_WARPS * 32>>>(
         H, q, zs, zx, zy, zz, idx, to_dev(p), force_order);
     return s.finish();
 }
@@ -1106,8 +1187,10 @@ static int do_grid_vanilla(SE_FGG_work* w, const SE_state* st, const SE_FGG_para
     const double* q = (const double*)s.use(st->q, 8 * (size_t)p->N, true, false);
     const double* zs = (const double*)s.use(w->zs, P3 * 8, true, false);
     SE_TRY(s.copy_in());
-    k_grid_vanilla<<<blocks(p->N, SCATTER_WARPS), SCATTER_WARPS * 32>>>(H, x, q, zs, to_dev(p),
-                                                                               periodicity_default());
+    const bool spread = scatter_vanilla_spread(p);
+    (spread ? k_grid_vanilla<true> : k_grid_vanilla<false>)<<<spread ? p->N : blocks(p->N, SCATTER_WARPS),
+                                                              SCATTER_WARPS * 32>>>(H, x, q, zs, to_dev(p),
+                                                                                    periodicity_default());
     return s.finish();
 }
 
@@ -1137,6 +1220,13 @@ static int do_extend(SE_FGG_work* w, const double* H_per, const SE_FGG_params* p
     return s.finish();
 }
 
+// Whether a gather walks the stencil's cells in order (SMALL_STENCIL): where its rows
+// leave lanes idle, P < 8, and P = 9, for which the row walk's 96 registers cost more
+// than its three rows of nine lanes gain (120,000 particles, M = 60, force: P = 4 211
+// -> 85 us, P = 6 327 -> 141, P = 9 411 -> 352; P = 10 488 by rows, 456 in order, its
+// potential 308 and 339; P = 13 682 and 878).
+static bool small_walk(const SE_FGG_params* p) { return p->P < 8 || p->P == 9; }
+
 static int do_int_split(double* phi, const SE_FGG_work* w, const SE_FGG_params* p,
                         bool accumulate)
 {
@@ -1160,6 +1250,7 @@ static int do_int_split(double* phi, const SE_FGG_work* w, const SE_FGG_params* 
     const auto fn = p->P == 16   ? k_int_split<16>
                     : p->P == 12 ? k_int_split<12>
                     : p->P == 8  ? k_int_split<8>
+                    : small_walk(p) ? k_int_split<SMALL_STENCIL>
                                  : k_int_split<0>;
     fn<<<blocks(p->N, 8), 256>>>(ph, H, zs, zx, zy, zz, idx, to_dev(p), h3, accumulate, order);
     return s.finish();
@@ -1212,6 +1303,7 @@ static int do_int_split_force(double* force, const SE_state* st, const SE_FGG_wo
     const auto fn = p->P == 16   ? k_int_split_force<16>
                     : p->P == 12 ? k_int_split_force<12>
                     : p->P == 8  ? k_int_split_force<8>
+                    : small_walk(p) ? k_int_split_force<SMALL_STENCIL>
                                  : k_int_split_force<0>;
     fn<<<blocks(p->N, 8), 256>>>(f, q, H, zs, zx, zy, zz, fx, fy, fz, idx, to_dev(p), h3, order);
     return s.finish();
