@@ -1110,17 +1110,25 @@ static bool grouped(const SE_FGG_params* p)
     return p->P >= 8 && (double)p->N * p->P * p->P * p->P >= 1.6e7;
 }
 
-// Whether a scatter goes through shared-memory windows: where they have far
-// fewer cells to clear and add than the particles' stencils (P = 16, all step
-// calls of a pass: 4,200 particles, M = 48, 2.8 times fewer, 337 -> 289 us;
-// 60,000, M = 128, 3.5 times, 2,053 -> 965 us; 6,000, M = 64, P = 12, 1.5 times,
-// no gain), and not where one window fills an SM (10,000, M = 45, P = 20, 5.6
-// times fewer: 814 us, without 614).
+// Whether a scatter goes through shared-memory windows: for many particles of a wide
+// stencil, or of one that is compiled in.  Scatter call, us, uniform and clustered
+// (sigma 0.004) particles, M = 60 and 48, straight into H and through windows:
+//   P = 16   15,000: 151, 201 and 161, 212;    40,000: 339, 472 and 292, 315
+//   P = 12   40,000: 170, 245 and 246, 275;   120,000: 438, 624 and 482, 490
+//   P = 8   120,000: 178, 257 and 228, 223;   500,000: 705, 1035 and 676, 649
+//   P = 15   40,000: 313, 366 and 345, 417;   120,000: 853, 1240 and 793, 815
+//   P = 13  120,000: 594, 794 and 692, 708
+//   P = 10  120,000: 292, 485 and 581, 642;   500,000: 1020, 1860 and 2652, 2637
+//   P = 6   500,000: 540, 646 and 1666, 1558
+// (a particle takes a CTA about a microsecond whatever P is).  Not where the windows'
+// cells are not far fewer than the stencils', nor where one window fills an SM
+// (10,000, M = 45, P = 20, all step calls of a pass: 814 us, without 614).
 static bool windowed(const SE_FGG_params* p, const StencilBins& B)
 {
-    const double W = p->P + BIN - 1, P = p->P;
-    return grouped(p) && p->P <= WINDOW_MAX_P &&
-           W * W * W * B.count * 2.0 < (double)p->N * P * P * P;
+    const double W = p->P + BIN - 1, P = p->P, cells = p->N * P * P * P;
+    const bool compiled = p->P == 8 || p->P == 12 || p->P == 16;
+    return p->P <= WINDOW_MAX_P && (compiled ? cells >= 1e8 : p->P >= 13 && cells >= 2.5e8) &&
+           W * W * W * B.count * 2.0 < cells;
 }
 
 // Whether a CTA, not a warp, scatters each particle: where a warp each would leave
