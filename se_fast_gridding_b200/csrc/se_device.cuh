@@ -70,7 +70,7 @@ __host__ __device__ inline bool spread2_general(int path, int M, int P)
 //   for potentials, gains nothing by it (P = 8 1.03 to 1.5x, P = 15 1.4 to 3x,
 //   P = 20 1.8 to 4.5x, potentials at P = 12 and 16 0.97 to 2x, forces there
 //   0.75 (120 per bin) to 1.5x (4 per bin)).
-__host__ __device__ inline bool interp3_better(int path, int precision, int M, int P, int mode)
+inline bool interp3_better(int path, int precision, int M, int P, int mode)
 {
     if (path & PATH_PAIR_INTERP)
         return precision == SE_FP64 && M >= (mode == SE_FORCE && P >= 10 && P <= 12 ? 192 : 128);
@@ -97,6 +97,7 @@ constexpr double PI_D = 3.14159265358979323846;
 struct SysDev {
     int N, M, P, lo, mode;
     int path;         // PATH_* bits
+    int interp3;      // k_interp3 serves the system (interp3_better)
     int part_off, out_off;
     long long grid_off, spec_off;
     int nf[3];        // fine bins per axis

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(INTERP_WARPS * 32) k_interp(
     const int beg = boff[bin], end = boff[bin + 1];
     if (beg == end) return;
     const SysDev& S = sys[find_sys(bin_prefix, nsys, bin)];
-    if ((S.path & PATH_PAIR_INTERP) || interp3_better(S.path, sizeof(T) == 4 ? SE_FP32 : SE_FP64, S.M, S.P, S.mode)) return;   // k_interp2, k_interp3
+    if ((S.path & PATH_PAIR_INTERP) || S.interp3) return;   // k_interp2, k_interp3
     const int P = PT ? PT : S.P;
     const int M = S.M;
     const int lb = bin - S.bin_base;

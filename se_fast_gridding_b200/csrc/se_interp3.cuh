@@ -125,8 +125,7 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
         sysi = find_sys(part_prefix, nsys, sperm[s0]);
         const SysDev& S = sys[sysi];
         if (S.P != P || S.mode != (FORCE ? SE_FORCE : SE_POTENTIAL) ||
-            ((S.path & PATH_PAIR_INTERP) != 0) != TILED ||
-            !interp3_better(S.path, sizeof(T) == 4 ? SE_FP32 : SE_FP64, S.M, S.P, S.mode))
+            ((S.path & PATH_PAIR_INTERP) != 0) != TILED || !S.interp3)
             return;   // another launch's system, or another kernel's
         const int pk = sg[s0];
         bin = S.bin_base + (g_of(pk, 0) / FB * S.nf[1] + g_of(pk, 1) / FB) * S.nf[2] + g_of(pk, 2) / FB;

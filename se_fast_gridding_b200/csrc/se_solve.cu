@@ -862,7 +862,7 @@ static int interp2_classes(se_batch_s* b, const se_system* systems, int nsys)
     int maxP = 0;
     for (int i = 0; i < nsys; i++) {
         const SysDev& S = b->host_sys[i];
-        const bool mma = interp3_better(S.path, b->precision, S.M, S.P, S.mode), tiled = S.path & PATH_PAIR_INTERP;
+        const bool mma = S.interp3, tiled = S.path & PATH_PAIR_INTERP;
         if (!mma && !tiled) continue;
         const bool any_p = b->runtime_p && !mma;
         Group& g = groups[{mma, tiled, any_p ? 0 : S.P, mma ? S.mode : SE_POTENTIAL}];
@@ -952,6 +952,7 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
         memset(&S, 0, sizeof(S));
         fill_sysdev(s, S);
         S.path = path_of(systems, paths, i);
+        S.interp3 = interp3_better(S.path, precision, S.M, S.P, S.mode);
         const int nf = S.nf[0];
         S.part_off = pcur;
         S.out_off = ocur;
@@ -1012,7 +1013,7 @@ static int batch_create(se_batch* out, const se_system* systems, int nsys, int p
         else b->any_spread1 = true;
         if (systems[i].N > split_cap(path, systems[i].M, systems[i].P, systems[i].N)) b->split = true;
         if (path & PATH_PAIR_INTERP) b->any_interp2 = true;
-        else if (const SysDev& S = b->host_sys[i]; !interp3_better(path, precision, S.M, S.P, S.mode)) {
+        else if (const SysDev& S = b->host_sys[i]; !S.interp3) {
             b->interp_P = !b->any_interp1 || b->interp_P == S.P ? S.P : 0;
             window_P = std::max(window_P, S.P);
             b->any_interp1 = true;
