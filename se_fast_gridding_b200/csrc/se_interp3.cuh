@@ -183,22 +183,22 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
             const double4 rc = srec[p];
             const int rx = g_of(pk, 0) - o0, ry = g_of(pk, 1) - o1, rz = g_of(pk, 2) - o2;
             double by[NK], fy[FORCE ? NK : 1];
-            const double uy = rc.y - (S.lo - ry) * h;
+            const double uy = fma(-(double)(S.lo - ry), h, rc.y);
 #pragma unroll
             for (int k = 0; k < NK; k++) {
                 by[k] = valid ? interp3_factor<TILED>(fac, PS, P, p, 1, 4 * k + t, ry, hy) : 0.0;
-                if (FORCE) fy[k] = by[k] * (-c * (uy - (4 * k + t) * h));
+                if (FORCE) fy[k] = by[k] * (-c * fma(-(double)(4 * k + t), h, uy));
             }
             int xlo = rx, xhi = rx + P;
             {
                 const int src = (lane & 7) * 4;
                 const int pn = __shfl_sync(0xffffffffu, p, src);
                 const int rn = __shfl_sync(0xffffffffu, rx, src);
-                const double ux = __shfl_sync(0xffffffffu, rc.x, src) - (S.lo - rn) * h;
+                const double ux = fma(-(double)(S.lo - rn), h, __shfl_sync(0xffffffffu, rc.x, src));
                 for (int x = lane >> 3; x < XE; x += 4) {
                     const double w = x < 4 * NK ? interp3_factor<TILED>(fac, PS, P, pn, 0, x, rn, hx) : 0.0;
                     wx[x][lane & 7] = w;
-                    if (FORCE) fx[x][lane & 7] = w * (-c * (ux - x * h));
+                    if (FORCE) fx[x][lane & 7] = w * (-c * fma(-(double)x, h, ux));
                 }
                 xlo = __reduce_min_sync(0xffffffffu, xlo);
                 xhi = __reduce_max_sync(0xffffffffu, xhi);
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
                 const int src = (2 * t + b) * 4;
                 pz[b] = __shfl_sync(0xffffffffu, p, src);
                 rzn[b] = __shfl_sync(0xffffffffu, rz, src);
-                uz[b] = __shfl_sync(0xffffffffu, rc.z, src) - (S.lo - rzn[b]) * h;
+                uz[b] = fma(-(double)(S.lo - rzn[b]), h, __shfl_sync(0xffffffffu, rc.z, src));
             }
             __syncwarp();
             const int ztop = __reduce_max_sync(0xffffffffu, rz) + P;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
                     if (FORCE) {
                         s[b][1] = fma(wz, ax[b], s[b][1]);
                         s[b][2] = fma(wz, ay[b], s[b][2]);
-                        s[b][3] = fma(wz * (-c * (uz[b] - z * h)), ap[b], s[b][3]);
+                        s[b][3] = fma(wz * (-c * fma(-(double)z, h, uz[b])), ap[b], s[b][3]);
                     }
                 }
             };
