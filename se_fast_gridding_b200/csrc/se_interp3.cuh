@@ -11,8 +11,8 @@
 // weighted with wx (and the force weights) and summed over the x planes in
 // the accumulators' own layout, then with wz.
 //
-// One CTA of 4 independent warps per bin (and per I3_PART further particles
-// of a crowded one); a warp takes a group at a time.  H comes straight from
+// One CTA of 4 independent warps per bin (and per `chunk` further particles
+// of a crowded one, launch_interp3); a warp takes a group at a time.  H comes straight from
 // the grid through L1: a window in shared memory (102 KB at P = 16, two CTAs
 // per SM) left the matrix unit idle while it was copied.  The operand tile is
 // laid so that its 8 rows are neighbouring z: a load touches 4 grid rows, and
@@ -38,7 +38,7 @@
 // spill).
 
 constexpr int I3_WARPS = 4;
-constexpr int I3_PART = 256;   // particles of a bin a CTA takes
+constexpr int I3_PART = 256;   // particles of a bin a CTA takes at most
 // from this many particles on they are grouped by whether they reach the last
 // z tile (with fewer, groups of 8 stay partly empty: 30 per bin, P = 12, 1.61
 // -> 1.78 ms)
@@ -94,12 +94,17 @@ __device__ __noinline__ double interp3_direct(const SysDev& S, const double* __r
     return sum;
 }
 
-// SHARE (launches of few bins): the z tiles of one or two groups go over all
-// the warps
+// CTAs per SM the kernel is compiled for: potentials of deep contractions do better with
+// the registers (200,000 particles, M = 100, potential, 7 and 5 CTAs: P = 20 482 and
+// 486 us, P = 24 618 and 587, P = 32 1137 and 1095; force, 4 and 3: P = 24 960 and 984)
+__host__ __device__ constexpr int interp3_ctas(int NK, bool force) { return force ? 4 : (NK >= 8 ? 5 : 7); }
+
+// SHARE (launches of few groups, in chunks of 8): the z tiles of one or two groups go
+// over all the warps
 template <int NK, bool FORCE, bool TILED, bool SHARE, typename T>
-__global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
+__global__ void __launch_bounds__(I3_WARPS * 32, interp3_ctas(NK, FORCE)) k_interp3(
     const SysDev* __restrict__ sys, const int* __restrict__ part_prefix, int nsys, const int* __restrict__ tab,
-    int units, int P, const double4* __restrict__ srec, const int* __restrict__ sg,
+    int units, int chunk, int P, const double4* __restrict__ srec, const int* __restrict__ sg,
     const int* __restrict__ sperm, const T* __restrict__ fac, int PS,
     const int* __restrict__ boff, const double* __restrict__ grid, double* __restrict__ out,
     double* __restrict__ phi_out)
@@ -111,17 +116,17 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
     __shared__ __align__(16) double wtab[I3_WARPS][FORCE ? 2 : 1][XE][8];   // the warps' x weights
     // the tiles' sums of every lane of shared groups
     __shared__ double part[SHARE ? 2 : 1][SHARE ? (NK + 1) / 2 : 1][FORCE ? 6 : 2][32];
-    // ---- the CTA's particles [c0, c0 + n) of one bin
+    // ---- the CTA's particles [c0, c0 + n) of one bin, at most `chunk`
     const int unit = blockIdx.x;
     int c0, n, sysi, bin;
     if (unit < units) {   // the first of unit's bin
         bin = __ldg(tab + units + unit);
         sysi = __ldg(tab + unit);
         c0 = boff[bin];
-        n = min(I3_PART, boff[bin + 1] - c0);
-    } else {   // of the sorted particles [s0, s0 + I3_PART) those past the
-               // first I3_PART of the bin that holds s0
-        const int s0 = (unit - units) * I3_PART;
+        n = min(chunk, boff[bin + 1] - c0);
+    } else {   // of the sorted particles [s0, s0 + chunk) those past the
+               // first `chunk` of the bin that holds s0
+        const int s0 = (unit - units) * chunk;
         sysi = find_sys(part_prefix, nsys, sperm[s0]);
         const SysDev& S = sys[sysi];
         if (S.P != P || S.mode != (FORCE ? SE_FORCE : SE_POTENTIAL) ||
@@ -129,8 +134,8 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
             return;   // another launch's system, or another kernel's
         const int pk = sg[s0];
         bin = S.bin_base + (g_of(pk, 0) / FB * S.nf[1] + g_of(pk, 1) / FB) * S.nf[2] + g_of(pk, 2) / FB;
-        c0 = max(boff[bin] + I3_PART, s0);
-        n = min(boff[bin + 1], s0 + I3_PART) - c0;
+        c0 = max(boff[bin] + chunk, s0);
+        n = min(boff[bin + 1], s0 + chunk) - c0;
     }
     if (n <= 0) return;
     const SysDev& S = sys[sysi];
@@ -371,6 +376,110 @@ __global__ void __launch_bounds__(I3_WARPS * 32, FORCE ? 4 : 7) k_interp3(
                 }
             }
             __syncwarp();   // the x weights are read before the next group's
+        }
+    }
+}
+
+// The same sums, a particle per warp: in sparse bins the groups above hold one or two
+// particles and cost as much as with 8.  A lane takes a z cell of the stencil and
+// walks its y and x cells in k_interp3's order (the cells it leaves out have zero
+// weights), so the results are the same bits.  Bound by the latency of its loads, 8
+// in flight (with 16, four planes at a time, N = 10,000, M = 100, P = 24 140 -> 176 us).
+template <bool FORCE, bool TILED, typename T>
+__global__ void __launch_bounds__(I3_WARPS * 32) k_interp3_sparse(
+    const SysDev* __restrict__ sys, const int* __restrict__ part_prefix, int nsys, int ntot, int P,
+    const double4* __restrict__ srec, const int* __restrict__ sg, const int* __restrict__ sperm,
+    const T* __restrict__ fac, int PS, const double* __restrict__ grid, double* __restrict__ out,
+    double* __restrict__ phi_out)
+{
+    constexpr int E = 40;   // cells of the widest window, whole z tiles
+    __shared__ double2 wxs[I3_WARPS][32], wys[I3_WARPS][32];   // weights, force weights
+    __shared__ int yos[I3_WARPS][32], xos[I3_WARPS][32];
+    __shared__ double sums[I3_WARPS][FORCE ? 3 : 1][E];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int p = blockIdx.x * I3_WARPS + warp;
+    if (p >= ntot) return;
+    const int orig = sperm[p];
+    const SysDev& S = sys[find_sys(part_prefix, nsys, orig)];
+    if (S.P != P || S.mode != (FORCE ? SE_FORCE : SE_POTENTIAL) || ((S.path & PATH_PAIR_INTERP) != 0) != TILED ||
+        !S.interp3)
+        return;
+    const int M = S.M, pk = sg[p];
+    const double4 rc = srec[p];
+    const double c = S.c, h = S.h;
+    const double* gs = grid + S.grid_off;
+    // the stencil's first cell in the bin's window, per axis
+    const int rx = g_of(pk, 0) % FB, ry = g_of(pk, 1) % FB, rz = g_of(pk, 2) % FB;
+    const int hx = g_of(pk, 0) - rx & 8, hy = g_of(pk, 1) - ry & 8, hz = g_of(pk, 2) - rz & 8;
+    if (lane < P) {
+        const int x = rx + lane, y = ry + lane;
+        const double wx = interp3_factor<TILED>(fac, PS, P, p, 0, x, rx, hx);
+        const double wy = interp3_factor<TILED>(fac, PS, P, p, 1, y, ry, hy);
+        const double ux = fma(-(double)(S.lo - rx), h, rc.x), uy = fma(-(double)(S.lo - ry), h, rc.y);
+        wxs[warp][lane] = make_double2(wx, wx * (-c * fma(-(double)x, h, ux)));
+        wys[warp][lane] = make_double2(wy, wy * (-c * fma(-(double)y, h, uy)));
+        xos[warp][lane] = (g_of(pk, 0) + lane) % M * M * M;
+        yos[warp][lane] = (g_of(pk, 1) + lane) % M * M;
+    }
+    for (int z = lane; z < E; z += 32)
+        for (int q = 0; q < (FORCE ? 3 : 1); q++) sums[warp][q][z] = 0.0;
+    __syncwarp();
+    if (lane < P) {
+        const double* col = gs + (g_of(pk, 2) + lane) % M;
+        double ap = 0, ax = 0, ay = 0;
+        for (int x = 0; x < P; x++) {
+            const double* plane = col + xos[warp][x];
+            double u = 0, v = 0;
+#pragma unroll 8
+            for (int y = 0; y < P; y++) {
+                const double cell = __ldg(plane + yos[warp][y]);
+                const double2 w = wys[warp][y];
+                u = fma(cell, w.x, u);
+                if (FORCE) v = fma(cell, w.y, v);
+            }
+            const double2 w = wxs[warp][x];
+            ap = fma(w.x, u, ap);
+            if (FORCE) {
+                ax = fma(w.y, u, ax);
+                ay = fma(w.x, v, ay);
+            }
+        }
+        sums[warp][0][rz + lane] = ap;
+        if (FORCE) {
+            sums[warp][FORCE ? 1 : 0][rz + lane] = ax;
+            sums[warp][FORCE ? 2 : 0][rz + lane] = ay;
+        }
+    }
+    __syncwarp();
+    // the sums over z: lane g < 8 the cells that k_interp3's lanes (g, t) hold, then the
+    // same halving
+    const int g = lane & 7, nz = (FB + P + 6) / 8, pairs = M % 2 == 0 ? nz / 2 : 0;
+    const double uz = fma(-(double)(S.lo - rz), h, rc.z);
+    double s[4] = {};
+    for (int i = 0; i < nz; i++) {
+        const int z = i < 2 * pairs ? 16 * (i / 2) + 2 * g + i % 2 : 8 * i + g;
+        const double wz = interp3_factor<TILED>(fac, PS, P, p, 2, z, rz, hz);
+        s[0] = fma(wz, sums[warp][0][z], s[0]);
+        if (FORCE) {
+            s[1] = fma(wz, sums[warp][FORCE ? 1 : 0][z], s[1]);
+            s[2] = fma(wz, sums[warp][FORCE ? 2 : 0][z], s[2]);
+            s[3] = fma(wz * (-c * fma(-(double)z, h, uz)), sums[warp][0][z], s[3]);
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < (FORCE ? 4 : 1); q++) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+    if (lane < (FORCE ? 4 : 1)) {
+        double val = lane == 0 ? s[0] : (lane == 1 ? s[1] : (lane == 2 ? s[2] : s[3]));
+        if (!isfinite(val)) val = interp3_direct<TILED>(S, gs, fac, PS, p, pk, rc, lane);
+        const int loc = orig - S.part_off;
+        const double scale = S.h3 * S.d;
+        if (lane == 0) {
+            double* dst = FORCE ? phi_out : out;
+            if (dst) dst[(FORCE ? S.part_off : S.out_off) + loc] = scale * val;
+        } else {
+            out[S.out_off + loc + (long long)(lane - 1) * S.N] = rc.w / S.d * scale * val;
         }
     }
 }

@@ -442,6 +442,7 @@ struct se_batch_s {
         bool tiled = false;     // from tile-aligned factor rows
         int mode = SE_POTENTIAL;   // k_interp3: the systems' mode
         int units = 0;          // CTAs: the systems' bins / zb
+        long long particles = 0;   // the systems' capacity
         int* tab = nullptr;     // device: each unit's system, then its first bin
     };
     std::vector<I2Class> i2_cls;
@@ -882,6 +883,7 @@ static int interp2_classes(se_batch_s* b, const se_system* systems, int nsys)
         c.P = std::get<2>(kv.first);
         c.mode = std::get<3>(kv.first);
         c.Pw = c.P ? c.P : maxP;
+        c.particles = kv.second.particles;
         if (c.mma) {
             c.zb = 1;
         } else {
@@ -1421,25 +1423,52 @@ static int launch_interp2(se_batch b, const T* grid, double* out, double* phi, c
                      : launch_interp2_mode<T, false>(b, grid, out, phi, st);
 }
 
-// Launches of at most this many bins (about four CTAs per SM) share a bin's z
-// tiles among the warps: 100 particles, M = 32, P = 21 27 -> 16 us with it; on
-// larger grids the repeated weights cost more than the idle warps.  The sums
-// are the same either way.
-constexpr int I3_SHARE_UNITS = 600;
+// How k_interp3's work is cut, by the size of the launch (the sums are the same
+// bits either way).  A group of 8 takes its warp long -- 5 z tiles of 39 planes at P = 32
+// -- and as long with one particle, so few particles go to as many warps as there are:
+// - launches of at most i3_share_groups groups (a bin each and every 8 particles) give
+//   a CTA one group, its z tiles shared by the warps;
+// - the others with at most i3_sparse_mean particles per bin and I3_SPARSE of them, go
+//   a particle per warp (k_interp3_sparse);
+// - up to I3_SMALL particles a CTA takes 32, a group per warp.
+// Interpolation stage, us, on FP64 FMAs (k_interp), with chunks of 256 always, and
+// now: 1,006 particles, M = 18, P = 32, force 100, 269, 68; 2,300, M = 155, P = 24,
+// force 111, 195, 88; 30,000 clustered, M = 100, P = 24, potential 1727, 393, 142.
+// 4,500 particles in 4,096 bins, P = 6, with shared groups 82, without 63.  Groups and
+// a particle per warp: 900, M = 100, P = 28, potential (shared) 70, 93, force 106, 98;
+// 5,000 in 2,197 bins, P = 24 106, 90, force 155, 123; 10,000 116, 140, force 177, 174.
+// From about 50,000 particles on groups are as good where they are sparse and better
+// where not (100,000 clustered, M = 250, P = 16, force 374, 624).
+constexpr int I3_SMALL = 40000;
+constexpr long long I3_SPARSE = 20000;
+static int i3_share_groups(bool force) { return force ? 900 : 1200; }
+static int i3_sparse_mean(bool force) { return force ? 4 : 3; }
 
 template <int NK, typename T>
 static int launch_interp3(se_batch b, const se_batch_s::I2Class& c, const double* grid, double* out,
                           double* phi, cudaStream_t st)
 {
     const bool force = c.mode == SE_FORCE;
-    const bool share = c.units <= I3_SHARE_UNITS;
+    const T* fac = static_cast<const T*>(c.tiled ? b->rows : b->fac);
+    const long long particles = std::min<long long>(c.particles, b->ntot);   // (a plan may hold fewer)
+    const bool share = std::min<long long>(c.units, particles) + particles / 8 <= i3_share_groups(force);
+    if (!share && particles <= std::min((long long)i3_sparse_mean(force) * c.units, I3_SPARSE)) {
+        const auto sparse = c.tiled ? (force ? k_interp3_sparse<true, true, T> : k_interp3_sparse<false, true, T>)
+                                    : (force ? k_interp3_sparse<true, false, T> : k_interp3_sparse<false, false, T>);
+        sparse<<<ceil_div(b->ntot, I3_WARPS), I3_WARPS * 32, 0, st>>>(
+            b->sys, b->d_part_prefix, b->nsys, b->ntot, c.P, b->srec, b->sg, b->perm, fac, b->PS, grid, out, phi);
+        SE_CUDA(cudaGetLastError());
+        LAUNCHED(b);
+        return SE_OK;
+    }
     auto fn = share ? (force ? k_interp3<NK, true, false, true, T> : k_interp3<NK, false, false, true, T>)
                     : (force ? k_interp3<NK, true, false, false, T> : k_interp3<NK, false, false, false, T>);
     if constexpr (NK <= interp3_nk(16) && sizeof(T) == 8)   // tile-aligned rows: FP64, P <= 16, larger grids
         if (c.tiled) fn = force ? k_interp3<NK, true, true, false, T> : k_interp3<NK, false, true, false, T>;
-    fn<<<c.units + ceil_div(b->ntot, I3_PART), I3_WARPS * 32, 0, st>>>(
-        b->sys, b->d_part_prefix, b->nsys, c.tab, c.units, c.P, b->srec, b->sg, b->perm,
-        static_cast<const T*>(c.tiled ? b->rows : b->fac), b->PS, b->boff, grid, out, phi);
+    const int chunk = share && !c.tiled ? 8 : (particles <= I3_SMALL ? 32 : I3_PART);
+    fn<<<c.units + ceil_div(b->ntot, chunk), I3_WARPS * 32, 0, st>>>(
+        b->sys, b->d_part_prefix, b->nsys, c.tab, c.units, chunk, c.P, b->srec, b->sg, b->perm, fac, b->PS,
+        b->boff, grid, out, phi);
     SE_CUDA(cudaGetLastError());
     LAUNCHED(b);
     return SE_OK;
