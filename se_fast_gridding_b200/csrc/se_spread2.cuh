@@ -338,17 +338,23 @@ struct Spread2Accum<double> {
                 *reinterpret_cast<double2*>(cell0 + 8 * h * plane + y * row) =
                     make_double2(v[y][2 * h], v[y][2 * h + 1]);
     }
-    // the same on a grid that may end inside the block (its rows of any alignment)
+    // the same on a grid that may end inside the block; of an odd one (row) the rows
+    // have any alignment, of an even one a lane's z and z + 1 are both on it or neither
     __device__ __forceinline__ void store(double* cell0, long long plane, int row, const BlockBounds& in) const
     {
+        const bool even = row % 2 == 0;
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
             for (int y = 0; y < 8; y++) {
                 double* c = cell0 + 8 * h * plane + y * row;
-                if (8 * h >= in.nx || y >= in.ny) continue;
-                if (in.nz > 0) c[0] = v[y][2 * h];
-                if (in.nz > 1) c[1] = v[y][2 * h + 1];
+                if (8 * h >= in.nx || y >= in.ny || in.nz <= 0) continue;
+                if (even) {
+                    *reinterpret_cast<double2*>(c) = make_double2(v[y][2 * h], v[y][2 * h + 1]);
+                } else {
+                    c[0] = v[y][2 * h];
+                    if (in.nz > 1) c[1] = v[y][2 * h + 1];
+                }
             }
     }
 };
@@ -565,21 +571,33 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     int* seg_beg = sm.seg_beg[lw];
     int* seg_pre = sm.seg_pre[lw];
     int total = 0;
-    for (int u0 = 0; u0 < nseg; u0 += 32) {
-        const int u = u0 + lane;
-        int beg = 0, len = 0;
-        if (u < nseg) B.segment(S, boff, u, beg, len);
-        int incl = len;
+    {
+        constexpr int R = (s2_segs<GEN>() + 31) / 32;
+        int beg[R], len[R], any = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
+        for (int r = 0; r < R; r++) {   // (every load first)
+            beg[r] = len[r] = 0;
+            if (32 * r + lane < nseg) B.segment(S, boff, 32 * r + lane, beg[r], len[r]);
+            any |= len[r];
         }
-        if (u < nseg) {
-            seg_beg[u] = beg;
-            seg_pre[u] = total + incl - len;
+        if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                int incl = len[r];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (32 * r + lane < nseg) {
+                    seg_beg[32 * r + lane] = beg[r];
+                    seg_pre[32 * r + lane] = total + incl - len[r];
+                }
+                total += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        } else {
+            nseg = 0;
         }
-        total += __shfl_sync(0xffffffffu, incl, 31);
     }
     __syncwarp();   // the warps are independent from here on
 
@@ -699,24 +717,29 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
                     const bool on = i < n && (unsigned)j < (unsigned)P;
                     cp_async_one_or_zero(dst, rows + ((long long)e.x * 3 + a) * PS + (on ? j : 0), on);
                 };
-                if (cls == 0) {
+                // (of a short group no more rows than its sums take, a multiple of 4)
+                auto stage = [&](auto rows_used) {
+                    if (cls == 0) {
 #pragma unroll 4
-                    for (int i = lane >> 4; i < G; i += 2)
-                        copy(&st.px[i][s2_px<F, GEN>(i, lane & 15)], i, 0, lane & 7, lane & 8);
-                } else {
-                    const int k = 8 * (cls - 1) + (lane & 7);
+                        for (int i = lane >> 4; i < rows_used; i += 2)
+                            copy(&st.px[i][s2_px<F, GEN>(i, lane & 15)], i, 0, lane & 7, lane & 8);
+                    } else {
+                        const int k = 8 * (cls - 1) + (lane & 7);
 #pragma unroll 4
-                    for (int i = lane >> 3; i < G; i += 4) copy(&st.px[i][s2_px<F, GEN>(i, k)], i, 0, lane & 7, 8 * (cls - 1));
-                }
+                        for (int i = lane >> 3; i < rows_used; i += 4) copy(&st.px[i][s2_px<F, GEN>(i, k)], i, 0, lane & 7, 8 * (cls - 1));
+                    }
 #pragma unroll 4
-                for (int i = lane >> 3; i < G; i += 4) {
-                    copy(&st.py[i][s2_pz<F>(i, lane & 7)], i, 1, lane & 7, 16);
-                    copy(&st.pz[i][s2_pz<F>(i, lane & 7)], i, 2, lane & 7, 24);
-                }
-                if (lane < G) {
-                    const unsigned p = lane < n ? list[(head + lane) & (S2_LIST - 1)].x : 0u;
-                    cp_async8_or_zero(&st.q[lane], &srec[p].w, lane < n);
-                }
+                    for (int i = lane >> 3; i < rows_used; i += 4) {
+                        copy(&st.py[i][s2_pz<F>(i, lane & 7)], i, 1, lane & 7, 16);
+                        copy(&st.pz[i][s2_pz<F>(i, lane & 7)], i, 2, lane & 7, 24);
+                    }
+                    if (lane < rows_used) {
+                        const unsigned p = lane < n ? list[(head + lane) & (S2_LIST - 1)].x : 0u;
+                        cp_async8_or_zero(&st.q[lane], &srec[p].w, lane < n);
+                    }
+                };
+                if (n == G) stage(std::integral_constant<int, G>());
+                else stage((n + 3) & ~3);
             } else {
                 constexpr int C8 = 8 / V, C16 = 16 / V;   // pieces per 8 and 16 entries
                 if (cls == 0) {
@@ -808,6 +831,13 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     // ---- the lane's cells
     if constexpr (FOLD) {
         if (since_fold > 0 || !written) acc.fold(cell0, plane, !written);
+    } else if (GEN && total == 0 && ipart == 0) {
+        // a block without candidates: zeros, 4 rows of 8 cells at a time (on an
+        // almost empty grid the stores are the spread)
+        const int nx = min(16, M - x0), ny = min(8, M - y0 - 8 * wy), nz = min(8, M - z0 - 8 * wz);
+        double* block = gs + (long long)x0 * gplane + (long long)(y0 + 8 * wy) * M + z0 + 8 * wz;
+        for (int r = lane >> 3; r < 128; r += 4)
+            if (r >> 3 < nx && (r & 7) < ny && (lane & 7) < nz) block[(r >> 3) * gplane + (r & 7) * M + (lane & 7)] = 0.0;
     } else if (GEN) {
         // (a slab holds whole tiles)
         const int end = ipart == 0 ? M : nt * 16;
@@ -825,14 +855,26 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
         __syncthreads();
         if (folds) {
             __threadfence();
-            for (int c = t; c < 4096; c += S2_THREADS) {
-                const int x = c >> 8, y = (c >> 4) & 15, z = c & 15;
-                if (GEN && (x0 + x >= M || y0 + y >= M || z0 + z >= M)) continue;
-                double* gp = gs + (long long)(x0 + x) * gplane + (long long)(y0 + y) * M + z0 + z;
-                double v = __ldcg(gp);
-                for (int k = 0; k < nparts - 1; k++)
-                    v += __ldcg(slab + (long long)(slot0 + k) * 4096 + c);
-                *gp = v;
+            // (8 cells of a thread side by side: the loads' latency is the time)
+            for (int c0 = t; c0 < 4096; c0 += 8 * S2_THREADS) {
+                double v[8];
+                auto cell = [&](int j) -> double* {
+                    const int c = c0 + j * S2_THREADS, x = c >> 8, y = (c >> 4) & 15, z = c & 15;
+                    if (GEN && (x0 + x >= M || y0 + y >= M || z0 + z >= M)) return nullptr;
+                    return gs + (long long)(x0 + x) * gplane + (long long)(y0 + y) * M + z0 + z;
+                };
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const double* gp = cell(j);
+                    v[j] = gp ? __ldcg(gp) : 0.0;
+                }
+                const double* sp = slab + (long long)slot0 * 4096 + c0;
+                for (int k = 0; k < nparts - 1; k++, sp += 4096)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] += __ldcg(sp + j * S2_THREADS);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (double* gp = cell(j)) *gp = v[j];
             }
             if (t == 0) tile_done[tile] = 0;
         }
