@@ -571,7 +571,20 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     int* seg_beg = sm.seg_beg[lw];
     int* seg_pre = sm.seg_pre[lw];
     int total = 0;
-    {
+    auto scan = [&](int u, int beg, int len) {
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (u < nseg) {
+            seg_beg[u] = beg;
+            seg_pre[u] = total + incl - len;
+        }
+        total += __shfl_sync(0xffffffffu, incl, 31);
+    };
+    if constexpr (GEN) {
         constexpr int R = (s2_segs<GEN>() + 31) / 32;
         int beg[R], len[R], any = 0;
 #pragma unroll
@@ -580,23 +593,15 @@ __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
             if (32 * r + lane < nseg) B.segment(S, boff, 32 * r + lane, beg[r], len[r]);
             any |= len[r];
         }
-        if (__any_sync(0xffffffffu, any)) {
+        if (!__any_sync(0xffffffffu, any)) nseg = 0;
+        else
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                int incl = len[r];
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                if (32 * r + lane < nseg) {
-                    seg_beg[32 * r + lane] = beg[r];
-                    seg_pre[32 * r + lane] = total + incl - len[r];
-                }
-                total += __shfl_sync(0xffffffffu, incl, 31);
-            }
-        } else {
-            nseg = 0;
+            for (int r = 0; r < R; r++) scan(32 * r + lane, beg[r], len[r]);
+    } else {
+        for (int u0 = 0; u0 < nseg; u0 += 32) {
+            int beg = 0, len = 0;
+            if (u0 + lane < nseg) B.segment(S, boff, u0 + lane, beg, len);
+            scan(u0 + lane, beg, len);
         }
     }
     __syncwarp();   // the warps are independent from here on
