@@ -96,11 +96,13 @@ int se_plan_destroy(se_plan plan);
 /* Kernel paths (se_plan_create_ex): which spread and interpolation kernels a
  * plan runs.  SE_PATH_TILE_SPREAD and SE_PATH_PAIR_INTERP (the kernels that read
  * tile-aligned factor rows) need M a multiple
- * of 16, M >= 32 and P <= 16; SE_PATH_RUNTIME_P turns off the interpolation
- * kernels specialised for P = 8, 12, 16 (21).  SE_PATH_DEFAULT is what
+ * of 16, M >= 32 and P <= 16; SE_PATH_RUNTIME_P turns off the window
+ * interpolation kernels specialised for P = 8, 12, 16 (systems that the
+ * matrix interpolation serves -- FP64 on tile-aligned rows from M = 128 or 192 on,
+ * most systems off them -- run the same kernels with it).  SE_PATH_DEFAULT is what
  * se_plan_create does (the tile spread where it applies, the pair
  * interpolation there too from P = 8 on); SE_PATH_TUNE times
- * every valid path on the plan's configuration (synthetic uniform particles,
+ * every valid path of different kernels on the plan's configuration (synthetic uniform particles,
  * N = max_particles, at most 2^20) and keeps the fastest, remembered per
  * (M, P, mode, precision, power-of-two class of N) for the process and, with
  * the environment variable SE_GPU_TUNE_FILE set, in that file.  Every path
@@ -127,7 +129,7 @@ int se_plan_destroy(se_plan plan);
 /* Stage one window per fine bin in the pair interpolation instead of one per
  * two z-adjacent bins (the FP32 default where the larger window fits three
  * CTAs per SM); both sum the same cells in the same order, so the results
- * are identical. */
+ * are identical.  Without effect where the matrix interpolation serves. */
 #define SE_PATH_BIN_WINDOWS 32
 int se_plan_create_ex(se_plan* plan, const se_config* cfg, int path);
 /* The path the default choice gives a system of grid M and stencil P. */

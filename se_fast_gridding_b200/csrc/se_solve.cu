@@ -672,15 +672,17 @@ static int batch_free(se_batch b)
 }
 
 // The k_interp kernel of a batch: specialised on P when all its systems have
-// the same and none asks for the runtime-P variants.
+// the same and none asks for the runtime-P variants (in FP64 it serves P <= 8 alone:
+// interp3_better).
 template <typename T>
 static const void* interp_kernel(const se_batch_s* b)
 {
     const int P = b->runtime_p ? 0 : b->interp_P;
-    return P == 8    ? (const void*)k_interp<T, 8>
-           : P == 12 ? (const void*)k_interp<T, 12>
-           : P == 16 ? (const void*)k_interp<T, 16>
-                     : (const void*)k_interp<T, 0>;
+    if constexpr (sizeof(T) == 4) {
+        if (P == 12) return (const void*)k_interp<T, 12>;
+        if (P == 16) return (const void*)k_interp<T, 16>;
+    }
+    return P == 8 ? (const void*)k_interp<T, 8> : (const void*)k_interp<T, 0>;
 }
 
 // Dynamic shared memory a kernel may use is a per-device, per-function
@@ -1809,18 +1811,19 @@ void tune_store(const TuneKey& k, int path)
     fclose(fp);
 }
 
-int tune_candidates(int M, int P, int* c)
+// The paths worth timing: SE_PATH_RUNTIME_P only where a window kernel with the stencil
+// compiled in serves the system without it (elsewhere both run the same kernels).
+int tune_candidates(const se_config& cfg, int* c)
 {
-    if (!spread2_eligible(M, P)) {
-        c[0] = 0;
-        c[1] = PATH_RUNTIME_P;
-        return 2;
+    const int precision = cfg.precision == SE_FP32_FFT32 ? SE_FP32 : cfg.precision;
+    const bool compiled = cfg.P == 8 || cfg.P == 12 || cfg.P == 16;
+    int n = 0;
+    for (int path : {PATH_TILE_SPREAD | PATH_PAIR_INTERP, PATH_TILE_SPREAD, PATH_PAIR_INTERP, 0}) {
+        if (path && !spread2_eligible(cfg.M, cfg.P)) continue;
+        c[n++] = path;
+        if (compiled && !interp3_better(path, precision, cfg.M, cfg.P, cfg.mode)) c[n++] = path | PATH_RUNTIME_P;
     }
-    const int all[6] = {PATH_TILE_SPREAD | PATH_PAIR_INTERP,
-                        PATH_TILE_SPREAD | PATH_PAIR_INTERP | PATH_RUNTIME_P,
-                        PATH_TILE_SPREAD, PATH_PAIR_INTERP, 0, PATH_RUNTIME_P};
-    for (int i = 0; i < 6; i++) c[i] = all[i];
-    return 6;
+    return n;
 }
 
 // Milliseconds of the fastest of 5 solves (after 2 untimed) on path `path`.
@@ -1858,8 +1861,12 @@ int tune_path(const se_config* cfg, int* path_out)
         *path_out = it->second;
         return SE_OK;
     }
-    int cand[6];
-    const int nc = tune_candidates(cfg->M, cfg->P, cand);
+    int cand[8];
+    const int nc = tune_candidates(*cfg, cand);
+    if (nc == 1) {
+        *path_out = g_tune[key] = cand[0];
+        return SE_OK;
+    }
     se_system s = sys_of(cfg, N);
     double *x = nullptr, *q = nullptr, *out = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
