@@ -61,10 +61,12 @@ __host__ __device__ inline bool spread2_general(int path, int M, int P)
 // PATH_PAIR_INTERP, k_interp without).  Measured on B200, interpolation stage:
 // - FP64 on tile-aligned rows: from M = 128 on, forces of P = 10 to 12 from M =
 //   192 on (M = 192, 1 to 80 particles per bin: 1.2 to 2.4x faster at P = 8 and
-//   16, potentials at P = 12 1.2 to 1.7x, forces at P = 12 0.96 to 1.1x); on
+//   16, potentials at P = 12 1.2 to 1.7x, forces at P = 12 0.96 to 1.1x; M = 128 to
+//   176, P = 8, 12 and 16, 0.5 to 40 per bin: no call slower); on
 //   smaller grids its warps are too few for their latency (M = 64: 0.7 to 1.1x);
 // - on other grids not for P <= 8 below M = 64 (M = 36, 1 to 18 per bin: 0.75
-//   to 1x, 4 us of a solve of 85);
+//   to 1x, 4 us of a solve of 85, with chunks of 256 particles; as its work is cut
+//   now, 4,500, M = 54, P = 8, force 48 and 52 us, crowded bins would gain);
 // - else FP64: always (M = 36 to 150, 1 to 120 per bin: 0.9 to 8x);
 // - else FP32: where the window kernel has no compiled-in stencil or,
 //   for potentials, gains nothing by it (P = 8 1.03 to 1.5x, P = 15 1.4 to 3x,

@@ -32,10 +32,12 @@
 // -> 0.139 ms; 2M clustered, M = 256, P = 12, force 3.34 -> 2.14 ms; 250,000,
 // M = 192, P = 12, potential 0.385 -> 0.305 ms; 1M, M = 256, P = 12, force 1.53
 // -> 1.55 ms, P = 8 potential 0.81 -> 0.49 ms.  At P = 16 the matrix unit is
-// 54% busy (its instructions alone take 0.126 ms), the load pipe 60%; the warps
+// 54% busy (its instructions alone take 0.126 ms), the L1 wavefronts 70%; the warps
 // in flight matter most (potentials with 4, 5 and 7 CTAs per SM at 250,000, P =
 // 12: 0.449, 0.315 and 0.305 ms; forces keep 128 registers, with fewer they
-// spill).
+// spill).  The weights are explicit FMAs, which every instantiation rounds alike (the
+// same products left to the compiler: 0.256 ms for 0.258 here, 0.104 for 0.101 at M =
+// 100, P = 12, and other last bits at P = 31 and 32 with shared groups).
 
 constexpr int I3_WARPS = 4;
 constexpr int I3_PART = 256;   // particles of a bin a CTA takes at most

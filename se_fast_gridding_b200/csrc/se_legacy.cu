@@ -349,7 +349,7 @@ __device__ int expand_one(const double xn[3], double q, const ParamsDev& p, int 
 // axes' powers side by side; the rows, which lie one after the other in memory,
 // go through shared memory and are stored 32 consecutive values at a time (by their own
 // lanes, P values apart, and row by row: call on 400,000 particles, P = 2, force, 55 and
-// 100 us, now 57; 1,000, P = 4 39, 47 and 41; 30,600, P = 16, force 61, 49 and 49).
+// 100 us, now 57; 1,000, P = 4 39, 47 and 41; 30,600, P = 16, force 60, 49 and 44).
 static size_t expand_bytes(int P) { return sizeof(double) * 3 * 32 * (size_t)(P | 1); }
 
 __global__ void __launch_bounds__(32) k_expand_all(

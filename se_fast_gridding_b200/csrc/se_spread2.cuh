@@ -110,7 +110,7 @@ constexpr int S2_CLASSES = 3;
 constexpr int S2_UNROLL = SE_S2_UNROLL;   // particles per unrolled pass of a group
 // FP32 CTAs per SM the kernel is compiled for: 5 (96 registers) where the
 // tiles outnumber 4 CTAs per SM, 4 (128 registers) where all of them are
-// resident at once either way; FP64: 3
+// resident at once either way; FP64 sums: 4
 constexpr int S2_BLOCKS_MANY = 5, S2_BLOCKS_FEW = 4, S2_BLOCKS_FP64 = 4;
 
 // particles a warp stages at once: one per lane (FP32 sums), half a warp (FP64)
@@ -507,8 +507,9 @@ __global__ void __launch_bounds__(TP_WARPS * 32) k_tile_parts(
 // 0.069 ms, P = 12 0.292 -> 0.110, P = 24 0.837 -> 0.379; 3,900, P = 8 0.023 ->
 // 0.016; 122,000, M = 250, P = 12 0.483 -> 0.183; 41,000, M = 128, P = 21 0.391 ->
 // 0.142.  FP32 0.131 -> 0.071, 0.238 -> 0.115, 0.627 -> 0.396, 0.021 -> 0.016,
-// 0.265 -> 0.185, 0.215 -> 0.146.  45 particles, M = 36:
-// 0.012 -> 0.013.  5,100, M = 32, P = 21 FP64 0.770 -> 0.467.
+// 0.265 -> 0.185, 0.215 -> 0.146.  5,100, M = 32, P = 21 FP64 0.770 -> 0.467 (in parts
+// 0.122).  Spread calls (sort and launches in them) of few particles: 53, M = 32, P =
+// 24 39 -> 41 us, 12, M = 281, P = 28 FP32 105 -> 110, FP64 123 -> 111.
 template <typename F, int BLOCKS, bool GEN = false, int CW = s2_cta_warps<F, GEN>()>
 __global__ void __launch_bounds__(CW * 32, BLOCKS * (S2_WARPS / CW)) k_spread2(
     const SysDev* __restrict__ sys, const int* __restrict__ tile_sys,
