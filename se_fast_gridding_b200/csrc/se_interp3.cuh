@@ -386,7 +386,9 @@ __global__ void __launch_bounds__(I3_WARPS * 32, interp3_ctas(NK, FORCE)) k_inte
 // particles and cost as much as with 8.  A lane takes a z cell of the stencil and
 // walks its y and x cells in k_interp3's order (the cells it leaves out have zero
 // weights), so the results are the same bits.  Bound by the latency of its loads, 8
-// in flight (with 16, four planes at a time, N = 10,000, M = 100, P = 24 140 -> 176 us).
+// in flight: 2,300 particles, M = 250, P = 21, potential 123 us (the cells past a
+// multiple of 8 one after the other 169); with 16, four planes at a time, 10,000, M =
+// 100, P = 24 176 for 140.
 template <bool FORCE, bool TILED, typename T>
 __global__ void __launch_bounds__(I3_WARPS * 32) k_interp3_sparse(
     const SysDev* __restrict__ sys, const int* __restrict__ part_prefix, int nsys, int ntot, int P,
@@ -422,6 +424,8 @@ __global__ void __launch_bounds__(I3_WARPS * 32) k_interp3_sparse(
         wys[warp][lane] = make_double2(wy, wy * (-c * fma(-(double)y, h, uy)));
         xos[warp][lane] = (g_of(pk, 0) + lane) % M * M * M;
         yos[warp][lane] = (g_of(pk, 1) + lane) % M * M;
+    } else {
+        wys[warp][lane] = make_double2(0.0, 0.0);
     }
     for (int z = lane; z < E; z += 32)
         for (int q = 0; q < (FORCE ? 3 : 1); q++) sums[warp][q][z] = 0.0;
@@ -432,12 +436,16 @@ __global__ void __launch_bounds__(I3_WARPS * 32) k_interp3_sparse(
         for (int x = 0; x < P; x++) {
             const double* plane = col + xos[warp][x];
             double u = 0, v = 0;
-#pragma unroll 8
-            for (int y = 0; y < P; y++) {
-                const double cell = __ldg(plane + yos[warp][y]);
-                const double2 w = wys[warp][y];
-                u = fma(cell, w.x, u);
-                if (FORCE) v = fma(cell, w.y, v);
+            for (int y0 = 0; y0 < P; y0 += 8) {
+                double cell[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) cell[k] = y0 + k < P ? __ldg(plane + yos[warp][y0 + k]) : 0.0;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {   // (past the stencil: zero times zero)
+                    const double2 w = wys[warp][y0 + k];
+                    u = fma(cell[k], w.x, u);
+                    if (FORCE) v = fma(cell[k], w.y, v);
+                }
             }
             const double2 w = wxs[warp][x];
             ap = fma(w.x, u, ap);

@@ -1430,8 +1430,10 @@ static int launch_interp2(se_batch b, const T* grid, double* out, double* phi, c
 // -- and as long with one particle, so few particles go to as many warps as there are:
 // - launches of at most i3_share_groups groups (a bin each and every 8 particles) give
 //   a CTA one group, its z tiles shared by the warps;
-// - the others with at most i3_sparse_mean particles per bin and I3_SPARSE of them, go
-//   a particle per warp (k_interp3_sparse);
+// - the others with at most i3_sparse_mean particles per bin and I3_SPARSE of them go
+//   a particle per warp (k_interp3_sparse), and those in 4,096 bins and more, 16 a
+//   particle, whose CTAs would nearly all return at once (67 particles, M = 280, P = 8,
+//   FP32 force 95, 54);
 // - up to I3_SMALL particles a CTA takes 32, a group per warp.
 // Interpolation stage, us, on FP64 FMAs (k_interp), with chunks of 256 always, and
 // now: 1,006 particles, M = 18, P = 32, force 100, 269, 68; 2,300, M = 155, P = 24,
@@ -1454,7 +1456,8 @@ static int launch_interp3(se_batch b, const se_batch_s::I2Class& c, const double
     const T* fac = static_cast<const T*>(c.tiled ? b->rows : b->fac);
     const long long particles = std::min<long long>(c.particles, b->ntot);   // (a plan may hold fewer)
     const bool share = std::min<long long>(c.units, particles) + particles / 8 <= i3_share_groups(force);
-    if (!share && particles <= std::min((long long)i3_sparse_mean(force) * c.units, I3_SPARSE)) {
+    const bool empty = c.units >= 4096 && 16 * particles <= c.units;   // nearly all CTAs of a launch by bins return at once
+    if (empty || (!share && particles <= std::min((long long)i3_sparse_mean(force) * c.units, I3_SPARSE))) {
         const auto sparse = c.tiled ? (force ? k_interp3_sparse<true, true, T> : k_interp3_sparse<false, true, T>)
                                     : (force ? k_interp3_sparse<true, false, T> : k_interp3_sparse<false, false, T>);
         sparse<<<ceil_div(b->ntot, I3_WARPS), I3_WARPS * 32, 0, st>>>(
